@@ -94,7 +94,7 @@ void Slot::release_buffers() {
   tiles.clear();
   tile_lru.clear();
   for (DevBuf* b : {&filt_Rf, &filt_ir2, &filt_np, &g_a, &g_D, &g_f, &chi, &stage, &counters, &ctl, &hdr, &geo, &pool, &okey,
-                    &okey2, &oidx, &oidx2, &otmp, &tcen, &tcount, &t_aos, &t_lapd, &mlim, &anchors, &mr_in, &mr_out, &mr_aux,
+                    &okey2, &oidx, &oidx2, &otmp, &tcen, &tcount, &t_aos, &t_lapd, &woff, &mlim, &anchors, &mr_in, &mr_out, &mr_aux,
                     &mr_rec, &mr_axis, &mr_amp, &pft})
     b->release();
   tune_save.release();
@@ -110,7 +110,7 @@ size_t Slot::bytes_held() const {
 size_t Slot::shell_bytes() const {
   size_t b = 0;
   for (const DevBuf* d : {&filt_Rf, &filt_ir2, &filt_np, &g_a, &g_D, &g_f, &chi, &stage, &counters, &ctl, &hdr, &geo, &pool,
-                          &okey, &okey2, &oidx, &oidx2, &otmp, &tcen, &tcount, &t_aos, &t_lapd, &mlim, &anchors, &mr_in,
+                          &okey, &okey2, &oidx, &oidx2, &otmp, &tcen, &tcount, &t_aos, &t_lapd, &woff, &mlim, &anchors, &mr_in,
                           &mr_out, &mr_aux, &mr_rec, &mr_axis, &mr_amp, &pft})
     b += d->bytes;
   if (iso) b += iso->bytes();

@@ -9,9 +9,8 @@
 // values sit n^2 apart; 16 consecutive y of one kx are one 128-byte segment)
 // and keeps the rows of four consecutive z planes in shared memory, so the
 // 3 x 3 x 3 maximum test runs on chip and the smoothed field never goes to
-// HBM.  The k^2-weighted twin (ioutshear) is
-// only needed at the peaks: its value there is a direct (n/2+1)-term sum over
-// its z/y-transformed row, in FP64.
+// HBM.  The k^2-weighted twin (ioutshear) is only needed at the peaks
+// (k_fft.cu).
 //
 // Real inverse DFT of length n = 64 J (unnormalised, Hermitian input X[0..H],
 // H = n/2): with Z[k] = (X[k] + conj X[H-k]) + i w^k (X[k] - conj X[H-k]),
@@ -200,8 +199,7 @@ struct XpArgs {
   const float2* ds;    // z/y-transformed smoothed field, [kx][z][y], kx <= n/2
   const float2* tw;    // w^k, k < n
   uint8_t* mask;       // n^3, x fastest
-  unsigned* first;     // lowest slot this launch appends (reset to ~0 before it)
-  int n, nbuff, tz, lap0;   // lap0: write lap = 0 (no k^2-weighted twin)
+  int n, nbuff, tz;
   float fcrit;
   unsigned long long keyhi;
   PeakBuf pb;
@@ -261,10 +259,7 @@ __global__ void __launch_bounds__(kXpThreads, 1) xpeak_kernel(XpArgs a) {
   auto flush = [&]() {
     __syncwarp();
     int base = 0;
-    if (l == 0) {
-      base = atomicAdd(a.pb.count, wn);
-      atomicMin(a.first, (unsigned)base);
-    }
+    if (l == 0) base = atomicAdd(a.pb.count, wn);
     base = __shfl_sync(full, base, 0);
     for (int e = l; e < wn; e += 32) {
       const int slot = base + e;
@@ -272,7 +267,7 @@ __global__ void __launch_bounds__(kXpThreads, 1) xpeak_kernel(XpArgs a) {
         a.pb.keys[slot] = (a.keyhi << 40) | (unsigned long long)myloc[e];
         a.pb.vals[slot] = (uint32_t)slot;
         a.pb.ff[slot] = myf[e];
-        if (a.lap0) a.pb.lap[slot] = 0.f;
+        a.pb.lap[slot] = 0.f;
       }
     }
     __syncwarp();
@@ -335,38 +330,6 @@ __global__ void __launch_bounds__(kXpThreads, 1) xpeak_kernel(XpArgs a) {
   if (wn > 0) flush();
 }
 
-// the k^2-weighted twin at the peaks one xpeak launch appended (slots
-// first .. count - 1): sum over kx of c_k Re(L[kx] w^(kx x)), c = 1 at kx = 0
-// and n/2, else 2, over the z/y-transformed twin in [kx][z][y] order; one warp
-// per peak
-__global__ void __launch_bounds__(256) lapsum_kernel(const float2* __restrict__ ls, const float2* __restrict__ tw,
-                                                    int n, const unsigned* __restrict__ first, PeakBuf pb) {
-  const unsigned f0 = *first;
-  if (f0 == 0xffffffffu) return;
-  const int end = (int)min((int64_t)*pb.count, pb.cap);
-  const int l = threadIdx.x & 31;
-  const int nw = gridDim.x * (blockDim.x / 32);
-  const int H = n / 2;
-  const int64_t nn = (int64_t)n * n;
-  for (int p = (int)f0 + blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5); p < end; p += nw) {
-    const long long loc = (long long)(pb.keys[p] & ((1ull << 40) - 1));
-    const int x = (int)(loc % n), y = (int)((loc / n) % n);
-    const long long z = loc / nn;
-    const float2* col = ls + n * z + y;
-    double acc = 0.0;
-#pragma unroll 4
-    for (int k = l; k <= H; k += 32) {
-      const float2 v = __ldg(col + nn * k);
-      const float2 t = __ldg(tw + (int)(((long long)k * x) % n));
-      const double term = (double)v.x * t.x - (double)v.y * t.y;
-      acc += (k == 0 || k == H) ? term : 2.0 * term;
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if (l == 0) pb.lap[p] = (float)acc;
-  }
-}
-
 // tw[k] = exp(2 pi i k / n) in float, from FP64 sincospi
 __global__ void twiddle_kernel(float2* tw, int n) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
@@ -377,12 +340,11 @@ __global__ void twiddle_kernel(float2* tw, int n) {
 }
 
 // window multiply of the filter bank (window_kernel's arithmetic) writing
-// the outputs transposed to [kx][kz][ky]: 32 x 32 (ky, kx) tiles of one kz
+// the output transposed to [kx][kz][ky]: 32 x 32 (ky, kx) tiles of one kz
 // plane through shared memory, both sides in 256-byte rows
-__global__ void __launch_bounds__(256) window_t_kernel(const float2* __restrict__ dk, float2* __restrict__ out0,
-                                                      float2* __restrict__ out1, int n,
+__global__ void __launch_bounds__(256) window_t_kernel(const float2* __restrict__ dk, float2* __restrict__ out, int n,
                                                       const float* __restrict__ tab, float ps) {
-  __shared__ float2 t0[32][33], t1[32][33];
+  __shared__ float2 t0[32][33];
   const int nh = n / 2 + 1, nyq = n / 2;
   const int kx0 = blockIdx.x * 32, ky0 = blockIdx.y * 32, kz = blockIdx.z;
   const int fz = kz <= nyq ? kz : kz - n;
@@ -390,30 +352,25 @@ __global__ void __launch_bounds__(256) window_t_kernel(const float2* __restrict_
   const int kx = kx0 + tx;
   if (kx < nh) {
     // the four loads and table lookups of this thread in flight together
-    float2 d[4], w[4];
+    float2 d[4];
+    float w[4];
 #pragma unroll
     for (int u = 0; u < 4; u++) {
       const int ky = ky0 + ty + 8 * u;
       const int fy = ky <= nyq ? ky : ky - n;
       d[u] = __ldg(dk + ((int64_t)kz * n + ky) * nh + kx);
-      w[u] = __ldg(reinterpret_cast<const float2*>(tab) + (kx * kx + fy * fy + fz * fz));
+      w[u] = __ldg(tab + 2 * (kx * kx + fy * fy + fz * fz));
     }
 #pragma unroll
-    for (int u = 0; u < 4; u++) {
-      const int r = ty + 8 * u;
-      t0[r][tx] = make_float2(__fmul_rn(__fmul_rn(d[u].x, w[u].x), ps), __fmul_rn(__fmul_rn(d[u].y, w[u].x), ps));
-      if (out1)
-        t1[r][tx] = make_float2(__fmul_rn(__fmul_rn(d[u].x, w[u].y), ps), __fmul_rn(__fmul_rn(d[u].y, w[u].y), ps));
-    }
+    for (int u = 0; u < 4; u++)
+      t0[ty + 8 * u][tx] = make_float2(__fmul_rn(__fmul_rn(d[u].x, w[u]), ps), __fmul_rn(__fmul_rn(d[u].y, w[u]), ps));
   }
   __syncthreads();
 #pragma unroll
   for (int cx = ty; cx < 32; cx += 8) {
     const int k = kx0 + cx;
     if (k >= nh) break;
-    const int64_t o = ((int64_t)k * n + kz) * n + ky0 + tx;
-    out0[o] = t0[tx][cx];
-    if (out1) out1[o] = t1[tx][cx];
+    out[((int64_t)k * n + kz) * n + ky0 + tx] = t0[tx][cx];
   }
 }
 
@@ -451,10 +408,9 @@ bool xpeak_supported(int n, int nbuff) {
   return n % 64 == 0 && n >= 64 && n <= 512 && nbuff >= 1 && n - 2 * nbuff >= 1;
 }
 
-void launch_window_t(Launch L, const float2* dk, float2* out0, float2* out1, int n, const float* tab,
-                     double post_scale) {
+void launch_window_t(Launch L, const float2* dk, float2* out, int n, const float* tab, double post_scale) {
   const dim3 grid((unsigned)((n / 2 + 1 + 31) / 32), (unsigned)(n / 32), (unsigned)n);
-  window_t_kernel<<<grid, dim3(32, 8), 0, L.s>>>(dk, out0, out1, n, tab, (float)post_scale);
+  window_t_kernel<<<grid, dim3(32, 8), 0, L.s>>>(dk, out, n, tab, (float)post_scale);
   PPB_LAUNCHED(*L.count);
 }
 
@@ -463,10 +419,9 @@ void launch_twiddles(Launch L, float2* tw, int n) {
   PPB_LAUNCHED(*L.count);
 }
 
-void launch_xpeak(Launch L, const float2* ds, const float2* ls, const float2* tw, uint8_t* mask, unsigned* first,
-                  int n, int nbuff, float fcrit, unsigned long long keyhi, PeakBuf pb) {
-  PPB_CUDA(cudaMemsetAsync(first, 0xff, sizeof(unsigned), L.s));
-  XpArgs a{ds, tw, mask, first, n, nbuff, 0, ls ? 0 : 1, fcrit, keyhi, pb};
+void launch_xpeak(Launch L, const float2* ds, const float2* tw, uint8_t* mask, int n, int nbuff, float fcrit,
+                  unsigned long long keyhi, PeakBuf pb) {
+  XpArgs a{ds, tw, mask, n, nbuff, 0, fcrit, keyhi, pb};
   switch (n / 64) {
     case 1: launch_j<1>(L, a); break;
     case 2: launch_j<2>(L, a); break;
@@ -477,10 +432,6 @@ void launch_xpeak(Launch L, const float2* ds, const float2* ls, const float2* tw
     case 7: launch_j<7>(L, a); break;
     case 8: launch_j<8>(L, a); break;
     default: PPB_REQUIRE(false, "fused x pass: unsupported grid size");
-  }
-  if (ls) {
-    lapsum_kernel<<<148 * 4, 256, 0, L.s>>>(ls, tw, n, first, pb);
-    PPB_LAUNCHED(*L.count);
   }
 }
 

@@ -171,7 +171,12 @@ void mr_tile_2lpt_lap(ppb_ctx* ctx, Slot& sl, TileRes& T, int n, double box, flo
     sl.launches++;
   };
   forward(T.delta.as<float>());
-  if (psi2) {
+  const bool fused = fft_supported(n);   // the fused transforms of k_fft.cu
+  if (psi2 && fused) {
+    float2* w[kLpt2Arrays];
+    fft_work_arrays(T, n, w);
+    launch_lpt2_fused(L, T.dk.as<float2>(), T.delta.as<float>(), w, T.xtw.as<float2>(), psi2, n, box, false);
+  } else if (psi2) {
     // phi_11, phi_22, phi_33, phi_12, phi_13, phi_23 (:812-821)
     const int pk6[6] = {3, 3, 3, 3, 3, 3}, pa[6] = {1, 2, 3, 1, 1, 2}, pb[6] = {1, 2, 3, 2, 3, 3};
     launch_kspace(L, nullptr, T.dk.as<float2>(), T.kw.as<float2>(), Mk, n, box, pk6, pa, pb, 6, post);
@@ -187,7 +192,11 @@ void mr_tile_2lpt_lap(ppb_ctx* ctx, Slot& sl, TileRes& T, int n, double box, flo
     PPB_CUFFT(cufftExecC2R(T.c2r3, T.kw.as<cufftComplex>() + Mk, psi2));
     sl.launches++;
   }
-  if (lapd) {
+  if (lapd && fused) {
+    const double dk = 2.0 * 3.141592653589793 / box;
+    launch_laplacian_fused(L, T.dk.as<float2>(), T.kw.as<float2>(), T.xtw.as<float2>(), lapd, n,
+                           (float)(dk * dk * post), true);
+  } else if (lapd) {
     const int k4[1] = {4}, z[1] = {0};
     launch_kspace(L, nullptr, T.dk.as<float2>(), T.kw.as<float2>(), Mk, n, box, k4, z, z, 1, post);
     PPB_CUFFT(cufftExecC2R(T.c2r1, T.kw.as<cufftComplex>(), lapd));

@@ -19,11 +19,11 @@ struct TileRes {
   int n = 0;
   cufftHandle r2c = 0, c2r1 = 0, c2r2 = 0, c2r3 = 0, c2r6 = 0;
   // in-place inverse C2C of contiguous n x n (kz, ky) planes, batched over
-  // the n/2+1 kx of one field (yz1) or of two fields back to back (yz2): the
-  // filter bank's transforms before the fused x pass (0 where unsupported)
-  cufftHandle yz1 = 0, yz2 = 0;
+  // the n/2+1 kx: the filter bank's transforms before the fused x pass (0
+  // where unsupported)
+  cufftHandle yz1 = 0;
   DevBuf delta, dk, psi, psi2, lapd, aos, kw, rw, mask, count, wtab;
-  DevBuf xtw;   // exp(2 pi i k / n), k < n: the fused x pass's twiddles
+  DevBuf xtw;   // exp(2 pi i k / n), k < n: twiddles of k_fft.cu and k_xpeak.cu (sizes of fft_supported)
   // peaks
   int64_t cap = 0;
   DevBuf keys, vals, ff, lap, keys_s, vals_s, tmp;
@@ -126,7 +126,7 @@ struct Slot {
   cudaTextureObject_t record_texture(const float4* aos, int n);
   void drop_record_texture();
   DevBuf okey, okey2, oidx, oidx2, otmp;            // spatial gather order
-  DevBuf tcen, tcount, t_aos, t_lapd;               // multi-tile: centres, peaks per tile, tile fields
+  DevBuf tcen, tcount, t_aos, t_lapd, woff;         // multi-tile: centres, peaks per tile, tile fields, window starts
   std::unique_ptr<IsoRes> iso;                      // multi-resolution: isolated convolution
   DevBuf mr_in, mr_out, mr_aux, mr_rec;             // multi-resolution: staged inputs, outputs, records
   DevBuf mr_axis, mr_amp;                           // multi-resolution: tricubic axis tables, coarse amplitudes
@@ -293,6 +293,8 @@ void peak_find_tile_core(ppb_ctx* ctx, Slot& sl, const float* delta, int n, cons
 // device, any may be null)
 void generate_fields_core(ppb_ctx* ctx, Slot& sl, const ppb_tile_params* p, float* delta, float* psi, float* psi2,
                           float* lapd);
+// the work arrays of launch_lpt2_fused: five in T.kw, four in T.rw
+void fft_work_arrays(TileRes& T, int n, float2** w);
 // device bytes a run of this grid size holds at most (admission estimate)
 uint64_t tile_footprint(const ppb_tile_params* p);
 // the part of it held per grid size (TileRes) and per slot (shell stage)

@@ -317,19 +317,47 @@ struct PeakBuf {
 // them); key = keyhi << 40 | (window-local flat index)
 void launch_peakfind(Launch L, const float* ds, const float* ls, uint8_t* mask, int n1, int n2, int n3,
                      int64_t py, int64_t pz, int nbuff, float fcrit, unsigned long long keyhi, PeakBuf pb);
-// the filter bank's x pass fused with the peak search (k_xpeak.cu): ds (and
-// ls) hold half spectra in [kx][z][y] order (window_t output) already
-// transformed back along z and y; one window over the whole n^3 grid.
+// the filter bank's x pass fused with the peak search (k_xpeak.cu): ds holds
+// a half spectrum in [kx][z][y] order (window_t output) already transformed
+// back along z and y; one window over the whole n^3 grid.
 // Supported for n = 64 J, J = 1..8, nbuff >= 1.
 bool xpeak_supported(int n, int nbuff);
 void xpeak_prepare(int n);
-void launch_window_t(Launch L, const float2* dk, float2* out0, float2* out1, int n, const float* tab,
-                     double post_scale);
+void launch_window_t(Launch L, const float2* dk, float2* out, int n, const float* tab, double post_scale);
 // tw[k] = exp(2 pi i k / n), k < n (the fused x pass's twiddles)
 void launch_twiddles(Launch L, float2* tw, int n);
-// first: device word the launch resets and lowers to the first slot it appends
-void launch_xpeak(Launch L, const float2* ds, const float2* ls, const float2* tw, uint8_t* mask, unsigned* first,
-                  int n, int nbuff, float fcrit, unsigned long long keyhi, PeakBuf pb);
+void launch_xpeak(Launch L, const float2* ds, const float2* tw, uint8_t* mask, int n, int nbuff, float fcrit,
+                  unsigned long long keyhi, PeakBuf pb);
+
+// transforms with fused k-space and real-space work (k_fft.cu), for grid
+// sizes 16 M with M up to 32 of factors 2, 3, 5, 7, 11 (fft_supported).  Rows
+// of the work arrays are fft_pitch(n) float2; tw[k] = exp(2 pi i k / n).
+bool fft_supported(int n);
+int fft_pitch(int n);
+int64_t fft_work_elems(int n);   // float2 of a work array
+void fft_prepare(int n);         // shared-memory opt-in, outside capture
+constexpr int kLpt2Arrays = 9;
+// psi2 (three n^3 fields) from dk = rfft(delta), Hermitian, and delta.  trace:
+// phi_33 from sum phi_aa = -delta (LPT.jl:86-191); else six phi without the
+// Nyquist planes and the trace-identity source (MultiResolution.jl:804-831).
+// w: kLpt2Arrays work arrays (arrays 5 and 8 are not used with trace)
+void launch_lpt2_fused(Launch L, const float2* dk, const float* delta, float2* const* w, const float2* tw, float* psi2,
+                       int n, double box, bool trace);
+// irfft(|f|^2 scale dk) (one work array)
+void launch_laplacian_fused(Launch L, const float2* dk, float2* w, const float2* tw, float* out, int n, float scale,
+                            bool zero_nyq);
+// z and y transforms of the k^2-weighted twins of `cnt` <= kTwinGroup
+// consecutive filters (window tables tab_stride floats apart) into w[i]
+// [z][y][kx], frequencies up to flim[i] = twin_flim(n, box, Rf); then their
+// values at the peaks of slots *first .. count - 1, whose keys hold the
+// filter (from f0) and the cell of an n1 x n2 window (starting at
+// woff[window], null: 0)
+constexpr int kTwinGroup = 8;
+int twin_flim(int n, double box, double Rf);
+void launch_twin_zy(Launch L, const float2* dk, float2* const* w, int cnt, const float2* tw, int n, const float* tab,
+                    int64_t tab_stride, float ps, const int* flim);
+void launch_twin_rows(Launch L, float2* const* w, int cnt, const float2* tw, int n, const int* flim, int n1, int n2,
+                      int fbits, int f0, const int64_t* woff, const int* first, PeakBuf pb);
 
 // Shell stage = five launches on one stream:
 //  geo      (one thread per peak): per-peak shell geometry

@@ -252,13 +252,13 @@ TileRes::~TileRes() {
   for (auto& g : graphs)   // before the plans whose kernels they launch
     if (g.second) cudaGraphExecDestroy(g.second);
   graphs.clear();
-  for (cufftHandle h : {r2c, c2r1, c2r2, c2r3, c2r6, yz1, yz2})
+  for (cufftHandle h : {r2c, c2r1, c2r2, c2r3, c2r6, yz1})
     if (h) cufftDestroy(h);
 }
 
 void TileRes::setup(int nn, cudaStream_t s) {
   if (n == nn) return;
-  for (cufftHandle* h : {&r2c, &c2r1, &c2r2, &c2r3, &c2r6, &yz1, &yz2})
+  for (cufftHandle* h : {&r2c, &c2r1, &c2r2, &c2r3, &c2r6, &yz1})
     if (*h) { cufftDestroy(*h); *h = 0; }
   n = nn;
   const int64_t N = (int64_t)n * n * n, M = (int64_t)(n / 2 + 1) * n * n;
@@ -278,6 +278,12 @@ void TileRes::setup(int nn, cudaStream_t s) {
   rw.ensure(6 * N * 4);
   mask.ensure(N);
   count.ensure(64);
+  if (fft_supported(n)) {   // the fused transforms' twiddles and shared-memory opt-in
+    fft_prepare(n);
+    xtw.ensure((size_t)n * sizeof(float2));
+    int64_t launched = 0;
+    launch_twiddles(Launch{s, &launched}, xtw.as<float2>(), n);
+  }
 }
 
 size_t TileRes::bytes() const {
@@ -289,15 +295,21 @@ size_t TileRes::bytes() const {
   return b;
 }
 
+// the work arrays of launch_lpt2_fused: five in T.kw, four in T.rw (32-byte
+// aligned: n is a multiple of 16)
+void fft_work_arrays(TileRes& T, int n, float2** w) {
+  const int64_t S = fft_work_elems(n);
+  PPB_REQUIRE((size_t)(5 * S * 8) <= T.kw.bytes && (size_t)(4 * S * 8) <= T.rw.bytes, "fused transforms: work arrays");
+  for (int i = 0; i < kLpt2Arrays; i++) w[i] = i < 5 ? T.kw.as<float2>() + i * S : T.rw.as<float2>() + (i - 5) * S;
+}
+
 void TileRes::setup_fused(cudaStream_t s) {
   if (yz1) return;
   int dims[2] = {n, n};
   const int nh = n / 2 + 1;
   PPB_CUFFT(cufftPlanMany(&yz1, 2, dims, nullptr, 1, 0, nullptr, 1, 0, CUFFT_C2C, nh));
-  PPB_CUFFT(cufftPlanMany(&yz2, 2, dims, nullptr, 1, 0, nullptr, 1, 0, CUFFT_C2C, 2 * nh));
-  for (cufftHandle h : {yz1, yz2}) PPB_CUFFT(cufftSetStream(h, s));
+  PPB_CUFFT(cufftSetStream(yz1, s));
   xpeak_prepare(n);
-  xtw.ensure((size_t)n * sizeof(float2));
 }
 
 void TileRes::ensure_peaks(int64_t c) {
@@ -489,8 +501,18 @@ void fields_phase(Run& r, TileRes& T, int n, double box) {
   } else {
     PPB_CUFFT(cufftExecC2R(T.c2r3, (cufftComplex*)kw, T.psi.as<cufftReal>()));
   }
+  // psi2 and the Laplacian feed no collapse decision: for the sizes of
+  // k_fft.cu they take the fused transforms (fields with 2LPT and Laplacian,
+  // all transforms by cuFFT -> these fused: 384^3 11.0 -> 7.2 ms, 352^3 9.9
+  // -> 6.2); elsewhere, and on the plain path, a full transform per field.
+  // delta and psi keep cuFFT's rounding, on which the peak list depends
+  const bool fused = !r.plain && fft_supported(n);
   // 2LPT
-  if (p->ilpt >= 2) {
+  if (p->ilpt >= 2 && fused) {
+    float2* w[kLpt2Arrays];
+    fft_work_arrays(T, n, w);
+    launch_lpt2_fused(L, dkp, T.delta.as<float>(), w, T.xtw.as<float2>(), T.psi2.as<float>(), n, box, true);
+  } else if (p->ilpt >= 2) {
     launch_phi(L, dkp, kw, n, box, inv_n3);
     launch_hermitise(L, kw, n, 6);
     if (r.plain) {
@@ -510,7 +532,11 @@ void fields_phase(Run& r, TileRes& T, int n, double box) {
     }
   }
   // Laplacian field (Pipeline.jl:35-51): irfft(k^2 delta_k) / n^3
-  if (r.want_lap) {
+  if (r.want_lap && fused) {
+    const double dk = 2.0 * 3.141592653589793 / box;
+    launch_laplacian_fused(L, dkp, kw, T.xtw.as<float2>(), T.lapd.as<float>(), n, (float)(dk * dk * inv_n3 * inv_n3),
+                           false);
+  } else if (r.want_lap) {
     launch_lapd(L, dkp, kw, n, box, (float)(inv_n3 * inv_n3));
     launch_hermitise(L, kw, n, 1);
     PPB_CUFFT(cufftExecC2R(T.c2r1, (cufftComplex*)kw, T.lapd.as<cufftReal>()));
@@ -545,6 +571,28 @@ int64_t peaks_phase(Run& r, TileRes& T, int n, double box, const std::vector<Win
   const bool fused = !r.plain && (fx == 1 || (fx == -1 && r.want_lap && (J & (J - 1)) != 0)) &&
                      xpeak_supported(n, p->nbuff) && wins.size() == 1 && wins[0].off == 0 && nm == n;
   if (fused) T.setup_fused(r.s);
+  // the k^2-weighted twin is read only at the peaks: for the sizes of
+  // k_fft.cu its z and y transforms alone (pruned to the frequencies its
+  // Gaussian window keeps) and one x sum per peak, after the search (20
+  // filters with the search, twin by full transforms -> this: 384^3 20.5 ->
+  // 18.2 ms, 352^3 34.3 -> 25.5, 192^3 2.85 -> 2.64)
+  const bool twin = r.want_lap && !r.plain && fft_supported(n);
+  // filters are taken in groups whose twin arrays together fit L2 (three
+  // launches per group; one filter at a time from 256^3 on)
+  const int64_t S = fft_work_elems(n);
+  const int group = std::max<int64_t>(1, std::min<int64_t>(kTwinGroup, ((int64_t)64 << 20) / (S * 8)));
+  float2* tw_w[kTwinGroup];   // behind the main field's spectrum and real field
+  for (int i = 0; i < kTwinGroup; i++)
+    tw_w[i] = i < 4 ? kw + M + i * S : reinterpret_cast<float2*>(rw + N) + (i - 4) * S;
+  PPB_REQUIRE(!twin || ((size_t)(M + 4 * S) * 8 <= T.kw.bytes && (size_t)N * 4 + (size_t)(4 * S) * 8 <= T.rw.bytes),
+              "twin work arrays");
+  int* first = T.count.as<int>() + 2;
+  if (twin && wins.size() > 1) {
+    std::vector<int64_t> woff;
+    for (const Win& w : wins) woff.push_back(w.off);
+    r.sl->woff.ensure(woff.size() * 8);
+    PPB_CUDA(cudaMemcpyAsync(r.sl->woff.p, woff.data(), woff.size() * 8, cudaMemcpyHostToDevice, r.s));
+  }
   int64_t npk = 0;
   for (int attempt = 0; attempt < 2; attempt++) {
     PeakBuf pb{T.keys.as<unsigned long long>(), T.vals.as<uint32_t>(), T.ff.as<float>(), T.lap.as<float>(),
@@ -557,30 +605,40 @@ int64_t peaks_phase(Run& r, TileRes& T, int n, double box, const std::vector<Win
       PPB_CUDA(cudaMemsetAsync(T.count.p, 0, 64, r.s));
       launch_window_tables(L, T.wtab.as<float>(), n, box, r.sl->filt_Rf.as<double>(), r.nfilt, p->wsmooth,
                            r.want_lap);
-      if (fused) launch_twiddles(L, T.xtw.as<float2>(), n);
       for (int f = 0; f < r.nfilt; f++) {
-        float2* o1 = r.want_lap ? kw + M : nullptr;
+        const float* tab = T.wtab.as<float>() + (size_t)f * 2 * qn;
+        if (twin && f % group == 0) PPB_CUDA(cudaMemcpyAsync(first, T.count.p, 4, cudaMemcpyDeviceToDevice, r.s));
         if (fused) {
-          // window multiply into [kx][kz][ky], z and y by cuFFT (both fields
-          // in one call), then x and the peak search in one kernel
-          launch_window_t(L, dkp, kw, o1, n, T.wtab.as<float>() + (size_t)f * 2 * qn, inv_n3);
-          PPB_CUFFT(cufftExecC2C(o1 ? T.yz2 : T.yz1, (cufftComplex*)kw, (cufftComplex*)kw, CUFFT_INVERSE));
-          launch_xpeak(L, kw, o1, T.xtw.as<float2>(), T.mask.as<uint8_t>(), T.count.as<unsigned>() + 2, n,
-                       p->nbuff, r.ffc.empty() ? wins[0].fcrit : r.ffc[f], (unsigned long long)f, pb);
-          continue;
-        }
-        launch_window(L, dkp, kw, o1, n, T.wtab.as<float>() + (size_t)f * 2 * qn, inv_n3);
-        if (r.want_lap && !r.plain) {
-          PPB_CUFFT(cufftExecC2R(T.c2r2, (cufftComplex*)kw, rw));
+          // window multiply into [kx][kz][ky], z and y by cuFFT, then x and
+          // the peak search in one kernel
+          launch_window_t(L, dkp, kw, n, tab, inv_n3);
+          PPB_CUFFT(cufftExecC2C(T.yz1, (cufftComplex*)kw, (cufftComplex*)kw, CUFFT_INVERSE));
+          launch_xpeak(L, kw, T.xtw.as<float2>(), T.mask.as<uint8_t>(), n, p->nbuff,
+                       r.ffc.empty() ? wins[0].fcrit : r.ffc[f], (unsigned long long)f, pb);
         } else {
-          PPB_CUFFT(cufftExecC2R(T.c2r1, (cufftComplex*)kw, rw));
-          if (r.want_lap) PPB_CUFFT(cufftExecC2R(T.c2r1, (cufftComplex*)(kw + M), rw + N));
+          const bool lap = r.want_lap && !twin;   // the full twin field, read by the search
+          launch_window(L, dkp, kw, lap ? kw + M : nullptr, n, tab, inv_n3);
+          if (lap && !r.plain) {
+            PPB_CUFFT(cufftExecC2R(T.c2r2, (cufftComplex*)kw, rw));
+          } else {
+            PPB_CUFFT(cufftExecC2R(T.c2r1, (cufftComplex*)kw, rw));
+            if (lap) PPB_CUFFT(cufftExecC2R(T.c2r1, (cufftComplex*)(kw + M), rw + N));
+          }
+          for (size_t t = 0; t < wins.size(); t++) {
+            const Win& w = wins[t];
+            launch_peakfind(L, rw + w.off, lap ? rw + N + w.off : nullptr, T.mask.as<uint8_t>() + w.off, nm, nm, nm,
+                            n, (int64_t)n * n, p->nbuff, r.ffc.empty() ? w.fcrit : r.ffc[f],
+                            ((unsigned long long)t << r.fbits) | (unsigned long long)f, pb);
+          }
         }
-        for (size_t t = 0; t < wins.size(); t++) {
-          const Win& w = wins[t];
-          launch_peakfind(L, rw + w.off, r.want_lap ? rw + N + w.off : nullptr, T.mask.as<uint8_t>() + w.off, nm,
-                          nm, nm, n, (int64_t)n * n, p->nbuff, r.ffc.empty() ? w.fcrit : r.ffc[f],
-                          ((unsigned long long)t << r.fbits) | (unsigned long long)f, pb);
+        if (twin && (f % group == group - 1 || f == r.nfilt - 1)) {
+          const int f0 = f / group * group, cnt = f - f0 + 1;
+          int flim[kTwinGroup];
+          for (int i = 0; i < cnt; i++) flim[i] = twin_flim(n, box, r.Rf[f0 + i]);
+          launch_twin_zy(L, dkp, tw_w, cnt, T.xtw.as<float2>(), n, T.wtab.as<float>() + (size_t)f0 * 2 * qn, 2 * qn,
+                         (float)inv_n3, flim);
+          launch_twin_rows(L, tw_w, cnt, T.xtw.as<float2>(), n, flim, nm, nm, r.fbits, f0,
+                           wins.size() > 1 ? r.sl->woff.as<int64_t>() : nullptr, first, pb);
         }
       }
     });
