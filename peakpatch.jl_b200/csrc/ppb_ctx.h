@@ -103,16 +103,16 @@ struct Slot {
   // merge_catalog's buffers, kept between calls (a cudaFree waits for the
   // whole device)
   struct MergeBufs {
-    DevBuf in, out, x, y, z, r, cell, cstart, cfill, cidx, rank, scount, sups, state, changed, rnew, key, key2, idx,
+    DevBuf in, out, x, y, z, r, cell, cstart, cfill, cidx, cpos, dV, rank, scount, sups, state, changed, rnew, key, key2, idx,
         idx2, tmp, flag, off, dom;
     void release() {
-      for (DevBuf* b : {&in, &out, &x, &y, &z, &r, &cell, &cstart, &cfill, &cidx, &rank, &scount, &sups, &state,
+      for (DevBuf* b : {&in, &out, &x, &y, &z, &r, &cell, &cstart, &cfill, &cidx, &cpos, &dV, &rank, &scount, &sups, &state,
                         &changed, &rnew, &key, &key2, &idx, &idx2, &tmp, &flag, &off, &dom})
         b->release();
     }
     size_t bytes() const {
       size_t t = 0;
-      for (const DevBuf* b : {&in, &out, &x, &y, &z, &r, &cell, &cstart, &cfill, &cidx, &rank, &scount, &sups, &state,
+      for (const DevBuf* b : {&in, &out, &x, &y, &z, &r, &cell, &cstart, &cfill, &cidx, &cpos, &dV, &rank, &scount, &sups, &state,
                               &changed, &rnew, &key, &key2, &idx, &idx2, &tmp, &flag, &off, &dom})
         t += b->bytes;
       return t;

@@ -231,9 +231,21 @@ __global__ void unpack_peaks_kernel(const unsigned long long* keys, int npk, int
   filt[q] = (int32_t)((key >> 40) & ((1ull << fbits) - 1)) + 1;
 }
 
-__global__ void tile_count_kernel(const unsigned long long* keys, int npk, int shift, int* counts) {
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q < npk) atomicAdd(counts + (int)(keys[q] >> shift), 1);
+// peaks per tile of the sorted keys (tile in the bits above shift): one
+// thread per tile, two binary searches (an atomic per peak on the few
+// counters took 0.3 ms for 0.4 M peaks)
+__global__ void tile_count_kernel(const unsigned long long* keys, int npk, int shift, int ntile, int* counts) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= ntile) return;
+  auto below = [&](unsigned long long v) {   // keys whose tile is below v
+    int lo = 0, hi = npk;
+    while (lo < hi) {
+      const int mid = (lo + hi) >> 1;
+      if ((keys[mid] >> shift) < v) lo = mid + 1; else hi = mid;
+    }
+    return lo;
+  };
+  counts[t] = below((unsigned long long)t + 1) - below((unsigned long long)t);
 }
 
 }  // namespace
@@ -1039,9 +1051,8 @@ void run_multitile_core(ppb_ctx* ctx, Slot& sl, const ppb_tile_params* p, const 
     while ((1 << tbits) < nwin) tbits++;
     PPB_CUDA(cudaMemsetAsync(T.count.p, 0, 64, r.s));
     sl.tcount.ensure(cnt.size() * 4);
-    PPB_CUDA(cudaMemsetAsync(sl.tcount.p, 0, cnt.size() * 4, r.s));
-    tile_count_kernel<<<(unsigned)((npk + 255) / 256), 256, 0, r.s>>>(T.keys_s.as<unsigned long long>(), (int)npk,
-                                                                      40 + r.fbits, sl.tcount.as<int>());
+    tile_count_kernel<<<(unsigned)((nwin + 63) / 64), 64, 0, r.s>>>(T.keys_s.as<unsigned long long>(), (int)npk,
+                                                                   40 + r.fbits, nwin, sl.tcount.as<int>());
     PPB_LAUNCHED(sl.launches);
     PPB_CUDA(cudaMemcpyAsync(cnt.data(), sl.tcount.p, cnt.size() * 4, cudaMemcpyDeviceToHost, r.s));
     PPB_CUDA(cudaStreamSynchronize(r.s));
