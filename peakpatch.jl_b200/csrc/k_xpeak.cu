@@ -206,6 +206,7 @@ struct XpArgs {
 };
 
 constexpr int kXpList = 64;   // per-warp peak list entries
+constexpr int kXpCells = 30;  // cells searched per warp step
 
 template <int J>
 __global__ void __launch_bounds__(kXpThreads, 1) xpeak_kernel(XpArgs a) {
@@ -279,7 +280,7 @@ __global__ void __launch_bounds__(kXpThreads, 1) xpeak_kernel(XpArgs a) {
   // (i + 1) & 1 and mask buffer (i + 1) & 1 are filled during iteration i.
   stage_plane(stg, z0 - 1);
   asm volatile("cp.async.commit_group;\n" ::);
-  const int W = hi - nb, nxc = (W + 31) / 32, nchunk = yi * nxc;
+  const int W = hi - nb, nxc = (W + kXpCells - 1) / kXpCells, nchunk = yi * nxc;
   for (int i = 0; i <= NP; i++) {
     asm volatile("cp.async.wait_all;\n" ::);
     __syncthreads();
@@ -297,23 +298,26 @@ __global__ void __launch_bounds__(kXpThreads, 1) xpeak_kernel(XpArgs a) {
     const float* s1 = ring + ((i - 2) & 3) * kXpRows * n;
     const float* s2 = ring + ((i - 1) & 3) * kXpRows * n;
     const uint8_t* mk = mbuf + (i & 1) * kXpInner * n;
-    // chunks of 32 cells of one row, spread over all warps
+    // chunks of 30 cells of one row (lanes 1..30; lanes 0 and 31 hold the
+    // neighbouring columns), spread over all warps.  A chunk with a candidate
+    // takes the maximum of the nine cells of its column per lane and the
+    // neighbours' by shuffle: nine shared-memory reads and no branch per
+    // chunk, where a test of the 27 cells one after another per candidate
+    // held a plane of a small radius (a fifth of the cells above fcrit) for
+    // several thousand cycles.  NaN compares as before: fmaxf drops it
     for (int ch = warp; ch < nchunk; ch += kXpThreads / 32) {
       const int ri = 1 + ch / nxc;
-      const int x = nb + 32 * (ch % nxc) + l;
+      const int x = nb - 1 + kXpCells * (ch % nxc) + l;
       const int y = y0 - 1 + ri;
-      bool peak = false;
-      float f = 0.f;
-      if (x < hi) {
-        f = s1[ri * n + x];
-        if (!(f < a.fcrit) && mk[(ri - 1) * n + x] != 1) {
-          peak = true;
-          for (int q = 0; q < 9; q++) {
-            const int o = (ri + q / 3 - 1) * n + x + q % 3 - 1;
-            if (f < s0[o] || f < s1[o] || f < s2[o]) { peak = false; break; }
-          }
-        }
-      }
+      const int o = ri * n + min(x, hi);
+      const float f = s1[o];
+      bool peak = l > 0 && l <= kXpCells && x < hi && !(f < a.fcrit) && mk[(ri - 1) * n + min(x, hi - 1)] != 1;
+      if (__ballot_sync(full, peak) == 0) continue;
+      float v = fmaxf(fmaxf(s1[o - n], f), s1[o + n]);
+      v = fmaxf(fmaxf(v, s0[o - n]), fmaxf(s0[o], s0[o + n]));
+      v = fmaxf(fmaxf(v, s2[o - n]), fmaxf(s2[o], s2[o + n]));
+      v = fmaxf(v, fmaxf(__shfl_up_sync(full, v, 1), __shfl_down_sync(full, v, 1)));
+      if (f < v) peak = false;
       const unsigned ball = __ballot_sync(full, peak);
       if (ball == 0) continue;
       if (peak) {
