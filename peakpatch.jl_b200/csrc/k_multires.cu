@@ -244,6 +244,56 @@ __global__ void __launch_bounds__(256) kspace_kernel(const float2* __restrict__ 
     if (s < sp.n) out[id + s * odist] = t[s];
 }
 
+// The transfer of the split's tile fields, kernels delta, psi_x, psi_y, psi_z
+// (kinds 0, 1, 1, 1) of the isolated box: kspace_kernel<true>'s arithmetic
+// with the kinds known at compile time, the threads flattened over a kz plane
+// and the mirror modes in their own branch.  Bound: FP64 conversions and
+// arithmetic next to HBM (8 bytes read, 32 written per mode; 0.17 ms at
+// 6.5 TB/s for a 384^3 box).  0.52 -> 0.26 ms per 384^3 box.
+__device__ __forceinline__ void field_modes(const float2* __restrict__ in, int n, int nh, int ix, int iy, int iz,
+                                            double mult, const double* __restrict__ amp_tab, float2 (&t)[4]) {
+  const float2 v = __ldg(in + ix + (int64_t)nh * (iy + (int64_t)n * iz));
+  const int fy = ifreq(iy, n), fz = ifreq(iz, n);
+  const double kx = (double)ix * mult, ky = (double)fy * mult, kz = (double)fz * mult;
+  const double k2 = kx * kx + ky * ky + kz * kz;
+  if (k2 == 0.0) {
+#pragma unroll
+    for (int s = 0; s < 4; s++) t[s] = make_float2(0.f, 0.f);
+    return;
+  }
+  const double amp = __ldg(amp_tab + (ix * ix + fy * fy + fz * fz));
+  const double inv_k2 = 1.0 / k2, a = (double)v.x, b = (double)v.y;
+  const double cx = amp * (kx * inv_k2), cy = amp * (ky * inv_k2), cz = amp * (kz * inv_k2);
+  t[0] = make_float2((float)(a * amp), (float)(b * amp));
+  t[1] = make_float2((float)(-b * cx), (float)(a * cx));
+  t[2] = make_float2((float)(-b * cy), (float)(a * cy));
+  t[3] = make_float2((float)(-b * cz), (float)(a * cz));
+}
+__global__ void __launch_bounds__(256) field_transfer_kernel(const float2* __restrict__ in, float2* __restrict__ out,
+                                                             int64_t odist, int n, double mult,
+                                                             const double* __restrict__ amp_tab) {
+  const int nh = n / 2 + 1, r = blockIdx.x * blockDim.x + threadIdx.x, iz = blockIdx.y;
+  if (r >= nh * n) return;
+  const int iy = r / nh, ix = r - iy * nh;
+  float2 t[4];
+  field_modes(in, n, nh, ix, iy, iz, mult, amp_tab, t);
+  if (ix == 0 || (n % 2 == 0 && ix == n / 2)) {
+    const int jy = (n - iy) % n, jz = (n - iz) % n;
+    if (jy == iy && jz == iz) {
+#pragma unroll
+      for (int s = 0; s < 4; s++) t[s].y = 0.f;
+    } else {
+      float2 u[4];
+      field_modes(in, n, nh, ix, jy, jz, mult, amp_tab, u);
+#pragma unroll
+      for (int s = 0; s < 4; s++) t[s] = make_float2(0.5f * (t[s].x + u[s].x), 0.5f * (t[s].y - u[s].y));
+    }
+  }
+  const int64_t id = r + (int64_t)nh * n * iz;
+#pragma unroll
+  for (int s = 0; s < 4; s++) out[id + s * odist] = t[s];
+}
+
 // ---------------------------------------------------------------------------
 // 2LPT source of run_multitile_split (:810-821):
 // src2 = d^2/2 - sum_a phi_aa^2/2 - sum_{a<b} phi_ab^2, each step rounded to
@@ -341,44 +391,101 @@ __device__ __forceinline__ void tri_load(const float* c, int q, float* v) {
   }
 }
 
+// val[u] (KZ cells of consecutive lk that share their four coarse planes kk):
+// the 64-term sums, each coarse value loaded once for the KZ cells
+template <int NF, int KZ>
+__device__ __forceinline__ void tri_sum(const float* coarse, const int4& ix, const int4& iy, const int4& iz,
+                                        const float (&wij)[4][4], const float4 (&wz)[KZ], int M,
+                                        float (&val)[KZ][NF]) {
+#pragma unroll
+  for (int u = 0; u < KZ; u++)
+#pragma unroll
+    for (int f = 0; f < NF; f++) val[u][f] = 0.0f;
+#pragma unroll
+  for (int a = 0; a < 4; a++) {
+#pragma unroll
+    for (int b = 0; b < 4; b++) {
+      const int row = M * (comp(iy, b) + M * comp(iz, a));
+#pragma unroll
+      for (int c = 0; c < 4; c++) {
+        float v[NF];
+        tri_load<NF>(coarse, row + comp(ix, c), v);
+#pragma unroll
+        for (int u = 0; u < KZ; u++) {
+          const float w3 = __fmul_rn(wij[b][c], comp(wz[u], a));
+          if constexpr (NF % 2 == 0) {   // two fields per instruction, each rounded as the scalar form
+#pragma unroll
+            for (int f = 0; f < NF; f += 2) {
+              const float2 p = __fmul2_rn(make_float2(w3, w3), make_float2(v[f], v[f + 1]));
+              const float2 s = __fadd2_rn(make_float2(val[u][f], val[u][f + 1]), p);
+              val[u][f] = s.x;
+              val[u][f + 1] = s.y;
+            }
+          } else {
+#pragma unroll
+            for (int f = 0; f < NF; f++) val[u][f] = __fadd_rn(val[u][f], __fmul_rn(w3, v[f]));
+          }
+        }
+      }
+    }
+  }
+}
+
+// A thread owns kTriZ cells of consecutive lk: they almost always lie in the
+// same coarse cell (a block of N / M fine cells), and the coarse values are
+// then loaded once for all (the loads bound the kernel: one cell per thread
+// took 0.35 ms for a 192^3 tile of four fields, this takes 0.18).  The planes of a
+// block's cells are the same for all its threads.
+constexpr int kTriZ = 4;
 template <int NF>
-__global__ void __launch_bounds__(128) tricubic_kernel(TriArgs<NF> A, const int4* __restrict__ aidx,
+__global__ void __launch_bounds__(64) tricubic_kernel(TriArgs<NF> A, const int4* __restrict__ aidx,
                                                        const float4* __restrict__ awt, int M, int n) {
   const int li = blockIdx.x * blockDim.x + threadIdx.x;
-  const int lj = blockIdx.y, lk = blockIdx.z;
+  const int lj = blockIdx.y, lk0 = blockIdx.z * kTriZ;
   if (li >= n) return;
-  const int4 ix = __ldg(aidx + li), iy = __ldg(aidx + n + lj), iz = __ldg(aidx + 2 * n + lk);
-  const float4 wx = __ldg(awt + li), wy = __ldg(awt + n + lj), wz = __ldg(awt + 2 * n + lk);
+  const int4 ix = __ldg(aidx + li), iy = __ldg(aidx + n + lj), iz = __ldg(aidx + 2 * n + lk0);
+  const float4 wx = __ldg(awt + li), wy = __ldg(awt + n + lj);
   // wi * wj for every (dii, djj): the first product of ((wi * wj) * wk) * f
   float wij[4][4];
 #pragma unroll
   for (int b = 0; b < 4; b++)
 #pragma unroll
     for (int c = 0; c < 4; c++) wij[b][c] = __fmul_rn(comp(wx, c), comp(wy, b));
-  float val[NF];
+  bool same = true;
+  float4 wz[kTriZ];
 #pragma unroll
-  for (int f = 0; f < NF; f++) val[f] = 0.0f;
+  for (int u = 0; u < kTriZ; u++) {
+    const int lk = min(lk0 + u, n - 1);
+    const int4 i2 = __ldg(aidx + 2 * n + lk);
+    same = same && i2.x == iz.x && i2.y == iz.y && i2.z == iz.z && i2.w == iz.w;
+    wz[u] = __ldg(awt + 2 * n + lk);
+  }
+  float val[kTriZ][NF];
+  if (same) {
+    tri_sum<NF, kTriZ>(A.coarse, ix, iy, iz, wij, wz, M, val);
+  } else {
+#pragma unroll 1
+    for (int u = 0; u < kTriZ; u++) {
+      const int lk = min(lk0 + u, n - 1);
+      const float4 w1[1] = {__ldg(awt + 2 * n + lk)};
+      float v1[1][NF];
+      tri_sum<NF, 1>(A.coarse, ix, iy, __ldg(aidx + 2 * n + lk), wij, w1, M, v1);
 #pragma unroll
-  for (int a = 0; a < 4; a++) {
-    const int kk = comp(iz, a);
-    const float wk = comp(wz, a);
+      for (int s = 0; s < kTriZ; s++)
+        if (s == u)
 #pragma unroll
-    for (int b = 0; b < 4; b++) {
-      const int row = M * (comp(iy, b) + M * kk);
-#pragma unroll
-      for (int c = 0; c < 4; c++) {
-        const float w3 = __fmul_rn(wij[b][c], wk);
-        float v[NF];
-        tri_load<NF>(A.coarse, row + comp(ix, c), v);
-#pragma unroll
-        for (int f = 0; f < NF; f++) val[f] = __fadd_rn(val[f], __fmul_rn(w3, v[f]));
-      }
+          for (int f = 0; f < NF; f++) val[s][f] = v1[0][f];
     }
   }
-  const int64_t o = li + (int64_t)n * (lj + (int64_t)n * lk);
-  const int64_t ob = A.bofs + li + A.bpy * lj + A.bpz * lk;
 #pragma unroll
-  for (int f = 0; f < NF; f++) A.out[f][o] = A.base[f] ? __fadd_rn(A.base[f][ob], val[f]) : val[f];
+  for (int u = 0; u < kTriZ; u++) {
+    const int lk = lk0 + u;
+    if (lk >= n) break;
+    const int64_t o = li + (int64_t)n * (lj + (int64_t)n * lk);
+    const int64_t ob = A.bofs + li + A.bpy * lj + A.bpz * lk;
+#pragma unroll
+    for (int f = 0; f < NF; f++) A.out[f][o] = A.base[f] ? __fadd_rn(A.base[f][ob], val[u][f]) : val[u][f];
+  }
 }
 
 // four M^3 fields a apart interleaved as float4 (the tricubic input of the
@@ -471,6 +578,14 @@ void launch_kspace(Launch L, const double* amp_tab, const float2* in, float2* ou
   PPB_LAUNCHED(*L.count);
 }
 
+void launch_field_transfer(Launch L, const double* amp_tab, const float2* in, float2* out, int64_t odist, int n,
+                           double box) {
+  const double dk = 2.0 * 3.141592653589793 / box;
+  const dim3 grid((unsigned)(((n / 2 + 1) * n + 255) / 256), (unsigned)n);
+  field_transfer_kernel<<<grid, 256, 0, L.s>>>(in, out, odist, n, ((double)n * dk) / (double)n, amp_tab);
+  PPB_LAUNCHED(*L.count);
+}
+
 void launch_src2_trace(Launch L, const float* delta, const float* phi, float* out, int n, int64_t px, int64_t pz,
                        int64_t pd) {
   dim3 grid((unsigned)((n + 127) / 128), (unsigned)n, (unsigned)n);
@@ -487,17 +602,17 @@ void launch_axis_weights(Launch L, int4* idx, float4* wt, int M, int64_t N, int6
 
 void launch_tricubic(Launch L, const int4* idx, const float4* wt, int M, int n, int nf, const float* coarse,
                      float* const* out, const float* const* base, int64_t bofs, int64_t bpy, int64_t bpz) {
-  dim3 grid((unsigned)((n + 127) / 128), (unsigned)n, (unsigned)n);
+  const dim3 grid((unsigned)((n + 63) / 64), (unsigned)n, (unsigned)((n + kTriZ - 1) / kTriZ));
   if (nf == 1) {
     TriArgs<1> A{coarse, {out[0]}, {base ? base[0] : nullptr}, bofs, bpy, bpz};
-    tricubic_kernel<1><<<grid, 128, 0, L.s>>>(A, idx, wt, M, n);
+    tricubic_kernel<1><<<grid, 64, 0, L.s>>>(A, idx, wt, M, n);
   } else if (nf == 4) {
     TriArgs<4> A{coarse,
                  {out[0], out[1], out[2], out[3]},
                  {base ? base[0] : nullptr, base ? base[1] : nullptr, base ? base[2] : nullptr,
                   base ? base[3] : nullptr},
                  bofs, bpy, bpz};
-    tricubic_kernel<4><<<grid, 128, 0, L.s>>>(A, idx, wt, M, n);
+    tricubic_kernel<4><<<grid, 64, 0, L.s>>>(A, idx, wt, M, n);
   } else {
     throw Error{PPB_ERR_INVALID, "tricubic: 1 or 4 fields per launch"};
   }

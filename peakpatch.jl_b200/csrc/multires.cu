@@ -219,9 +219,7 @@ void mr_split_tile_fields(ppb_ctx* ctx, Slot& sl, TileRes& T, const float* cnois
   iso_forward(sl, iso);
   // delta, psi_x, psi_y, psi_z of the isolated convolution (:740-752)
   const double box = (double)n2 * (box_local / (double)nm);
-  const int kind[4] = {0, 1, 1, 1}, d1[4] = {0, 1, 2, 3}, d2[4] = {0, 0, 0, 0};
-  launch_kspace(L, iso_amp(ctx, sl, iso, box), iso.spec.as<float2>(), iso.work.as<float2>(), modes, n2, box, kind, d1,
-                d2, 4, 1.0 / ((double)n2 * (double)n2 * (double)n2));
+  launch_field_transfer(L, iso_amp(ctx, sl, iso, box), iso.spec.as<float2>(), iso.work.as<float2>(), modes, n2, box);
   for (int q = 0; q < 4; q++) iso_inverse(sl, iso, iso.work.as<float2>() + q * modes, 0, nm);
   // plus the tricubic coarse fields, read from the transforms in place
   // (:764-795): one pass writes the four tile fields

@@ -417,6 +417,10 @@ void launch_amp_table(Launch L, double* tab, int n, double box, const double* lk
 // and Nyquist planes zeroed); Hermitian projection fused
 void launch_kspace(Launch L, const double* amp_tab, const float2* in, float2* out, int64_t odist, int n, double box,
                    const int* kind, const int* d1, const int* d2, int nspec, double post);
+// the kernels delta, psi_x, psi_y, psi_z of an n^3 box (launch_kspace's
+// transfer for kinds 0, 1, 1, 1)
+void launch_field_transfer(Launch L, const double* amp_tab, const float2* in, float2* out, int64_t odist, int n,
+                           double box);
 void launch_src2_trace(Launch L, const float* delta, const float* phi, float* out, int n, int64_t px, int64_t pz,
                        int64_t pd);
 // per-axis tricubic indices and weights (3n entries) of the n^3 tile at
