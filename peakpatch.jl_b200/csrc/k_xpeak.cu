@@ -229,27 +229,35 @@ __global__ void __launch_bounds__(kXpThreads, 1) xpeak_kernel(XpArgs a) {
   RowConsts<J> c;
   row_consts<J>(c, l, a.tw);
   // rows y0 - 1 .. y0 - 2 + R of plane z: per kx one contiguous run of R
-  // float2, two kx per warp step (half-warps)
-  auto stage_plane = [&](float2* stg, int z) {
-    const float2* src = a.ds + (int64_t)n * z + (y0 - 1);
-    const int r = l & 15;
-    for (int kx = 2 * warp + (l >> 4); kx < nh; kx += 2 * (kXpThreads / 32)) {
-      if (r < R) {
-        const unsigned dst = (unsigned)__cvta_generic_to_shared(stg + kx * kXpPad + r);
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(dst), "l"(src + nn * kx + r));
-      }
+  // float2, two kx per warp step (half-warps).  The kernel is issue-bound, so
+  // addresses advance by constants: kx = kx0 + 32 j, j < J, and kx = H
+  const int kx0 = 2 * warp + (l >> 4), rl = l & 15;
+  const float2* src0 = a.ds + nn * kx0 + (y0 - 1) + rl;
+  const unsigned dst0 = (unsigned)__cvta_generic_to_shared(stg + kx0 * kXpPad + rl);
+  auto stage_plane = [&](int buf, int z) {
+    const float2* src = src0 + n * z;
+    const unsigned dst = dst0 + buf * (nh * kXpPad * 8);
+    if (rl < R) {
+#pragma unroll
+      for (int j = 0; j < J; j++)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(dst + j * (32 * kXpPad * 8)),
+                     "l"(src + j * (32 * nn)));
+      if (kx0 == 0)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(dst + J * (32 * kXpPad * 8)),
+                     "l"(src + J * (32 * nn)));
     }
   };
-  // mask bytes of the inner rows of plane z, x in [nb, hi) rounded out to
-  // 4-byte words, into buf[row][x]
-  auto stage_mask = [&](uint8_t* buf, int z) {
-    const int w0 = nb >> 2, w1 = (hi + 3) >> 2;
-    const uint8_t* src = a.mask + nn * z + (int64_t)n * y0;
-    for (int r = warp; r < yi; r += kXpThreads / 32)
-      for (int w = w0 + l; w < w1; w += 32) {
-        const unsigned dst = (unsigned)__cvta_generic_to_shared(buf + r * n + 4 * w);
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(dst), "l"(src + (int64_t)n * r + 4 * w));
-      }
+  // mask bytes of the inner rows of plane z, x in [nb, hi) rounded out to 16
+  // bytes, into buf[row][x]: one warp per row (yi <= kXpInner < 16 warps, at
+  // most 32 pieces of 16 bytes)
+  const int mw = (nb >> 4) + l;
+  const bool mask_on = warp < yi && mw < (hi + 15) >> 4;
+  const uint8_t* msrc0 = a.mask + (int64_t)n * (y0 + warp) + 16 * mw;
+  const unsigned mdst0 = (unsigned)__cvta_generic_to_shared(mbuf + warp * n + 16 * mw);
+  auto stage_mask = [&](int buf, int z) {
+    if (mask_on)
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(mdst0 + buf * (kXpInner * n)),
+                   "l"(msrc0 + nn * z));
   };
   // this warp's peak list: appended without atomics, flushed to the peak
   // buffers (one atomicAdd) when it could overflow and at the end
@@ -278,14 +286,17 @@ __global__ void __launch_bounds__(kXpThreads, 1) xpeak_kernel(XpArgs a) {
   // buffer i & 1 into ring slot i & 3 while plane i - 2 is searched between
   // slots i - 3 and i - 1; one barrier per iteration.  Staging buffer
   // (i + 1) & 1 and mask buffer (i + 1) & 1 are filled during iteration i.
-  stage_plane(stg, z0 - 1);
+  stage_plane(0, z0 - 1);
   asm volatile("cp.async.commit_group;\n" ::);
-  const int W = hi - nb, nxc = (W + kXpCells - 1) / kXpCells, nchunk = yi * nxc;
+  // a row's chunks; chunk number warp, warp + 16, ... as (row, chunk of row)
+  constexpr int kWarps = kXpThreads / 32;
+  const int W = hi - nb, nxc = (W + kXpCells - 1) / kXpCells;
+  const int ri0 = warp / nxc, xc0 = warp - ri0 * nxc, dri = kWarps / nxc, dxc = kWarps - dri * nxc;
   for (int i = 0; i <= NP; i++) {
     asm volatile("cp.async.wait_all;\n" ::);
     __syncthreads();
-    if (i + 1 < NP) stage_plane(stg + ((i + 1) & 1) * nh * kXpPad, z0 + i);
-    if (i + 1 >= 3 && i + 1 <= NP) stage_mask(mbuf + ((i + 1) & 1) * kXpInner * n, z0 - 2 + i);
+    if (i + 1 < NP) stage_plane((i + 1) & 1, z0 + i);
+    if (i + 1 >= 3 && i + 1 <= NP) stage_mask((i + 1) & 1, z0 - 2 + i);
     asm volatile("cp.async.commit_group;\n" ::);
     if (i < NP && warp < R) {
       float2 x[J], xh;
@@ -305,13 +316,17 @@ __global__ void __launch_bounds__(kXpThreads, 1) xpeak_kernel(XpArgs a) {
     // chunk, where a test of the 27 cells one after another per candidate
     // held a plane of a small radius (a fifth of the cells above fcrit) for
     // several thousand cycles.  NaN compares as before: fmaxf drops it
-    for (int ch = warp; ch < nchunk; ch += kXpThreads / 32) {
-      const int ri = 1 + ch / nxc;
-      const int x = nb - 1 + kXpCells * (ch % nxc) + l;
-      const int y = y0 - 1 + ri;
+    for (int r = ri0, xc = xc0; r < yi; r += dri, xc += dxc) {
+      if (xc >= nxc) {
+        xc -= nxc;
+        if (++r >= yi) break;
+      }
+      const int ri = 1 + r;
+      const int x = nb - 1 + kXpCells * xc + l;
+      const int y = y0 + r;
       const int o = ri * n + min(x, hi);
       const float f = s1[o];
-      bool peak = l > 0 && l <= kXpCells && x < hi && !(f < a.fcrit) && mk[(ri - 1) * n + min(x, hi - 1)] != 1;
+      bool peak = l > 0 && l <= kXpCells && x < hi && !(f < a.fcrit) && mk[r * n + x] != 1;
       if (__ballot_sync(full, peak) == 0) continue;
       float v = fmaxf(fmaxf(s1[o - n], f), s1[o + n]);
       v = fmaxf(fmaxf(v, s0[o - n]), fmaxf(s0[o], s0[o + n]));
