@@ -590,9 +590,9 @@ int64_t peaks_phase(Run& r, TileRes& T, int n, double box, const std::vector<Win
   // 18.2 ms, 352^3 34.3 -> 25.5, 192^3 2.85 -> 2.64)
   const bool twin = r.want_lap && !r.plain && fft_supported(n);
   // filters are taken in groups whose twin arrays together fit L2 (three
-  // launches per group; one filter at a time from 256^3 on)
+  // launches per group), from 256^3 on in pairs that share their reads of dk
   const int64_t S = fft_work_elems(n);
-  const int group = std::max<int64_t>(1, std::min<int64_t>(kTwinGroup, ((int64_t)64 << 20) / (S * 8)));
+  const int group = std::max<int64_t>(2, std::min<int64_t>(kTwinGroup, ((int64_t)64 << 20) / (S * 8)));
   float2* tw_w[kTwinGroup];   // behind the main field's spectrum and real field
   for (int i = 0; i < kTwinGroup; i++)
     tw_w[i] = i < 4 ? kw + M + i * S : reinterpret_cast<float2*>(rw + N) + (i - 4) * S;
