@@ -20,12 +20,14 @@
 // Carlson RD evaluations of the shape integrals, within each the lanes x, y,
 // z (z twice) carry one component, so that a duplication's three square
 // roots, and its three divisions by the average, are one instruction
-// sequence; the four Lagrange weights of the growth table are one per lane.
-// The background at a step's end is the next step's start and the two
-// midpoint evaluations share theirs, so it is evaluated twice per step.
+// sequence, with lane 3's division for the series' sum beside them; the four
+// Lagrange weights of the growth table are one per lane, and so are the
+// divisions of the equations of motion.  The background at a step's end is
+// the next step's start and the two midpoint evaluations share theirs, so
+// both are evaluated once, side by side, at the step's start.
 // Nodes are taken by ascending F, the longest integrations first.  One thread
-// per node: 307 ms for the 50 x 20 x 20 table; this: 197 ms
-// (the same bits).
+// per node: 307 ms for the 50 x 20 x 20 table; this: 174 ms,
+// 107 ms of it the longest node's latency (the same bits).
 //
 // Bit-exactness with the CPU oracle: this file is compiled without
 // multiply-add contraction (-fmad=false), so that every +, -, *, / and sqrt
@@ -127,7 +129,7 @@ __device__ void rd2(double x, double y, double z, double u, double w, bool need,
   const int l = threadIdx.x & 31, base = l & 28, c = l & 3;
   const bool second = (l & 4) != 0;
   double t = c == 0 ? (second ? u : x) : c == 1 ? y : (second ? w : z);
-  double sum = 0.0, fac = 1.0, d = 0.0, ave = 1.0;   // sum is the z lanes'
+  double sum = 0.0, fac = 1.0, d = 0.0, ave = 1.0;   // sum is lane 3's
   bool go = need;
   for (int it = 0; it < 200; it++) {
     const double s = sqrt(t);
@@ -138,21 +140,21 @@ __device__ void rd2(double x, double y, double z, double u, double w, bool need,
     const double xt = __shfl_sync(kAll, tn, base), yt = __shfl_sync(kAll, tn, base + 1),
                  zt = __shfl_sync(kAll, tn, base + 2);
     const double an = 0.2 * (xt + yt + 3.0 * zt);
-    const double dn = (an - tn) / an;
-    const double q = fac / (s * (t + al));
+    // lanes 0-2 divide for the spread, lane 3 (z again) for the sum
+    const double dn = (c == 3 ? fac : an - tn) / (c == 3 ? s * (t + al) : an);
     if (go) {
-      sum += q;
+      sum += dn;
       fac *= 0.25;
       t = tn;
       ave = an;
       d = dn;
     }
-    const unsigned wide = __ballot_sync(kAll, go && !(fabs(d) <= ERRTOL));
+    const unsigned wide = __ballot_sync(kAll, go && c < 3 && !(fabs(d) <= ERRTOL));
     go = go && ((wide >> base) & 15u) != 0;
     if (wide == 0) break;
   }
   const double dx = __shfl_sync(kAll, d, base), dy = __shfl_sync(kAll, d, base + 1), dz = __shfl_sync(kAll, d, base + 2);
-  sum = __shfl_sync(kAll, sum, base + 2);
+  sum = __shfl_sync(kAll, sum, base + 3);
   const double ea = dx * dy, eb = dz * dz, ec = ea - eb, ed = ea - 6.0 * eb, ee = ed + ec + ec;
   const double r = 3.0 * sum + fac * (1.0 + ed * (-C1 + C5 * ed - C6 * dz * ee) + dz * (C2 * ee + dz * (-C3 * ec + dz * C4 * ea))) /
                           (ave * sqrt(ave));
@@ -160,11 +162,10 @@ __device__ void rd2(double x, double y, double z, double u, double w, bool need,
   *r2 = __shfl_sync(kAll, r, (l & 24) + 4);
 }
 
-// shape integrals b_1..b_3 of axes a1, a2, a3 (whole warps; live: the node
-// still integrates)
-__device__ void shape_b(double a1, double a2, double a3, bool live, double* b) {
+// shape integrals b_1..b_3 of the axis ratios r2 = a2 / a1, r3 = a3 / a1
+// (whole warps; live: the node still integrates)
+__device__ void shape_b(double r2, double r3, bool live, double* b) {
   const double third = 1.0 / 3.0;
-  const double r2 = a2 / a1, r3 = a3 / a1;
   const bool oblate = r3 >= r2;   // or spherical
   const double r22 = r2 * r2, r32 = r3 * r3, q = third * r2 * r3;
   double rd3, rd2v;
@@ -214,20 +215,25 @@ __device__ __forceinline__ double force(const TabArgs& A, const Ell& S, double y
   }
 }
 
-// the background at scale factor a: H and, for the external tidal forces that
+// the background at a scale factor: H and, for the external tidal forces that
 // use it, D
 struct Bg {
   double Ha, dl;
 };
-__device__ Bg background(const TabArgs& A, Ell& S, double a) {
-  Bg g;
-  g.Ha = hubble(A, a);
-  g.dl = 0.0;
+// at the midpoint (lanes 0-3 of a node) and the end (lanes 4-7) of a step
+__device__ void background2(const TabArgs& A, Ell& S, double mid, double end, Bg* gm, Bg* ge) {
+  const int l = threadIdx.x & 31, base = l & 24;
+  const double a = (l & 4) ? end : mid;
+  const double Ha = hubble(A, a);
+  double dl = 0.0;
   if (A.iforce == 4 || A.iforce == 5 || A.iforce == 6) {
     double hd;
-    dlin(A, a, &g.dl, &hd, &S.pos);
+    dlin(A, a, &dl, &hd, &S.pos);
   }
-  return g;
+  gm->Ha = __shfl_sync(kAll, Ha, base);
+  gm->dl = __shfl_sync(kAll, dl, base);
+  ge->Ha = __shfl_sync(kAll, Ha, base + 4);
+  ge->dl = __shfl_sync(kAll, dl, base + 4);
 }
 
 // get_derivs!: virialisation checks (axis 3 first), frozen axes written back
@@ -236,9 +242,7 @@ __device__ void derivs(const TabArgs& A, Ell& S, double t, const Bg& g, bool liv
 #pragma unroll
   for (int i = 0; i < 6; i++) dy[i] = 0.0;
   const double ab = t, ab3 = ab * ab * ab;
-  const double Ha = g.Ha;
-  S.Ha = Ha;
-  const double Hi = 1.0 / Ha;
+  S.Ha = g.Ha;
   if (S.lv2 == 0 && y[2] <= A.fcoll3 * ab) {
     S.lv2 = 1;
     S.eq2 = A.fcoll3 * ab;
@@ -252,22 +256,30 @@ __device__ void derivs(const TabArgs& A, Ell& S, double t, const Bg& g, bool liv
   if (S.lv1) { y[1] = S.eq1; y[4] = 0.0; }
   if (S.lv0) { y[0] = S.eq0; y[3] = 0.0; }
   const double a1 = y[0], a2 = y[1], a3 = y[2];
-  const double d1e = ab3 / (a1 * a2 * a3);
+  // the step's divisions, one per lane of the node, in two rounds
+  const int l = threadIdx.x & 31, base = l & 24, k = l & 7;
+  const double num = k == 0 ? 1.0 : k == 1 ? ab3 : k == 2 ? a2 : k == 3 ? a3 : k == 4 ? 0.5 : k == 5 ? 1.5 : 1.5 * 2.5;
+  const double den = k == 0 ? g.Ha : k == 1 ? a1 * a2 * a3 : k <= 3 ? a1 : ab3;
+  const double quo = num / den;
+  const double Hi = __shfl_sync(kAll, quo, base), d1e = __shfl_sync(kAll, quo, base + 1),
+               r2 = __shfl_sync(kAll, quo, base + 2), r3 = __shfl_sync(kAll, quo, base + 3),
+               half_ab3 = __shfl_sync(kAll, quo, base + 4), x3_ab3 = __shfl_sync(kAll, quo, base + 5),
+               x75_ab3 = __shfl_sync(kAll, quo, base + 6);
   double d0, d1i, d1x = 0.0;
   if (A.iforce == 0) {
     d0 = -A.Rvac * Hi;
     d1i = 1.5 * d1e / ab3 * Hi;
   } else {
-    d0 = (0.5 / ab3 - A.Rvac) * Hi;
+    d0 = (half_ab3 - A.Rvac) * Hi;
     d1i = 1.5 * (d1e - 1.0) / ab3 * Hi;
     if (A.iforce == 4 || A.iforce == 5 || A.iforce == 6) {
-      d1x = 1.5 / ab3 * Hi * g.dl;
+      d1x = x3_ab3 * Hi * g.dl;
     } else if (A.iforce == 3) {
-      d1x = 1.5 * 2.5 / ab3 * Hi;
+      d1x = x75_ab3 * Hi;
     }
   }
   double b[3] = {0.0, 0.0, 0.0};
-  if (A.iforce != 5 && A.iforce != 6) shape_b(a1, a2, a3, live, b);
+  if (A.iforce != 5 && A.iforce != 6) shape_b(r2, r3, live, b);
   if (!S.lv2) { dy[2] = y[5] * Hi; dy[5] = force(A, S, y[2], b[2], S.lam2, d0, d1i, d1x, ab); }
   if (!S.lv1) { dy[1] = y[4] * Hi; dy[4] = force(A, S, y[1], b[1], S.lam1, d0, d1i, d1x, ab); }
   if (!S.lv0) { dy[0] = y[3] * Hi; dy[3] = force(A, S, y[0], b[0], S.lam0, d0, d1i, d1x, ab); }
@@ -313,9 +325,10 @@ __global__ void __launch_bounds__(64, 8) table_kernel(TabArgs A) {
     istep += live;
     const double a_3 = y[2];
     const double h = A.tfac * a_3 * sqrt(a_3) * S.Ha;
-    derivs(A, S, t, g0, live, y, dy);
     const double hh = h * 0.5, h6 = h / 6.0, xh = t + hh;
-    const Bg gh = background(A, S, xh);
+    Bg gh, g1;
+    background2(A, S, xh, t + h, &gh, &g1);
+    derivs(A, S, t, g0, live, y, dy);
 #pragma unroll
     for (int c = 0; c < 6; c++) yt[c] = y[c] + hh * dy[c];
     derivs(A, S, xh, gh, live, yt, dyt);
@@ -327,8 +340,8 @@ __global__ void __launch_bounds__(64, 8) table_kernel(TabArgs A) {
       yt[c] = y[c] + h * dym[c];
       dym[c] = dyt[c] + dym[c];
     }
-    g0 = background(A, S, t + h);
-    derivs(A, S, t + h, g0, live, yt, dyt);
+    derivs(A, S, t + h, g1, live, yt, dyt);
+    g0 = g1;
     if (!live) continue;
 #pragma unroll
     for (int c = 0; c < 6; c++) y[c] = y[c] + h6 * (dy[c] + dyt[c] + 2.0 * dym[c]);
