@@ -87,9 +87,16 @@ cudaTextureObject_t Slot::record_texture(const float4* aos, int n) {
   return rec_tex;
 }
 
+// the record array of a stub call may be among them: its texture goes first
+void Slot::release_stub() {
+  drop_record_texture();
+  for (DevBuf& b : stub) b.release();
+}
+
 void Slot::release_buffers() {
   if (stream) PPB_CUDA(cudaStreamSynchronize(stream));
   drop_record_texture();
+  release_stub();
   merge.release();
   tiles.clear();
   tile_lru.clear();
@@ -113,6 +120,7 @@ size_t Slot::shell_bytes() const {
                           &okey, &okey2, &oidx, &oidx2, &otmp, &tcen, &tcount, &t_aos, &t_lapd, &woff, &mlim, &anchors, &mr_in,
                           &mr_out, &mr_aux, &mr_rec, &mr_axis, &mr_amp, &pft})
     b += d->bytes;
+  for (const DevBuf& d : stub) b += d.bytes;
   if (iso) b += iso->bytes();
   return b;
 }

@@ -87,6 +87,7 @@ struct ShellStats {
 // An execution slot: one CUDA stream and every buffer a tile run writes.
 // Runs on different slots overlap on the device; one slot runs one tile at a
 // time.
+constexpr size_t kStubKeep = (size_t)4 << 30;   // stub buffers kept between calls at most
 struct Slot {
   int device = 0;
   cudaStream_t stream = nullptr;
@@ -130,6 +131,8 @@ struct Slot {
   std::unique_ptr<IsoRes> iso;                      // multi-resolution: isolated convolution
   DevBuf mr_in, mr_out, mr_aux, mr_rec;             // multi-resolution: staged inputs, outputs, records
   DevBuf mr_axis, mr_amp;                           // multi-resolution: tricubic axis tables, coarse amplitudes
+  DevBuf stub[19];                                  // the stub entry points' staging and outputs (stubs.cu)
+  void release_stub();
   DevBuf pft;                                       // ppb_peak_find_tile: unpacked (i, j, k), ipp, filter
   int gather_bps[2][2][2] = {};                      // gather blocks per SM by [comp][adaptive][ring]
   double rows_per_peak[2] = {0.0, 0.0};             // pool rows per peak seen last, by adaptive

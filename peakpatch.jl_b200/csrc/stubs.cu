@@ -77,6 +77,24 @@ __global__ void skip_out_kernel(const int32_t* skip, int64_t nq, double* out) {
   o[26] = -1.0;
 }
 
+// The buffers of one stub call, kept in the slot between calls (a cudaMalloc
+// and cudaFree per buffer and call, each free waiting for the device, took 3
+// of the 9 ms of 200,000 peaks on a 256^3 grid); given back at the end of the
+// call when they hold more than kStubKeep bytes.  The caller holds ctx->mu,
+// and the call has waited for the stream when it ends without an error.
+struct StubCall {
+  Slot& sl;
+  explicit StubCall(Slot& s) : sl(s) {}
+  DevBuf& operator[](int i) { return sl.stub[i]; }
+  ~StubCall() {
+    size_t b = 0;
+    for (const DevBuf& d : sl.stub) b += d.bytes;
+    if (b <= kStubKeep) return;
+    cudaStreamSynchronize(sl.stream);
+    sl.release_stub();
+  }
+};
+
 }  // namespace
 
 extern "C" {
@@ -93,7 +111,10 @@ int32_t ppb_find_peaks(ppb_ctx* ctx, const float* delta, int8_t* mask, int32_t n
     cudaStream_t s = ctx->sync.stream;
     const int64_t N = (int64_t)n1 * n2 * n3;
     PPB_REQUIRE(N < (1ll << 40), "grid too large");
-    DevBuf d_delta, d_mask, keys, vals, ff, cnt, keys_s, vals_s, tmp, o_i, o_j, o_k, o_ipp, o_d;
+    StubCall call(ctx->sync);
+    DevBuf &d_delta = call[0], &d_mask = call[1], &keys = call[2], &vals = call[3], &ff = call[4], &cnt = call[5],
+           &keys_s = call[6], &vals_s = call[7], &tmp = call[8], &o_i = call[9], &o_j = call[10], &o_k = call[11],
+           &o_ipp = call[12], &o_d = call[13], &lapdummy = call[14];
     const float* dd = (const float*)[&]() -> const void* {
       if (is_device_ptr(delta)) return delta;
       d_delta.ensure(N * 4);
@@ -118,8 +139,6 @@ int32_t ppb_find_peaks(ppb_ctx* ctx, const float* delta, int8_t* mask, int32_t n
     PPB_CUDA(cudaMemsetAsync(cnt.p, 0, 64, s));
     PeakBuf pb{keys.as<unsigned long long>(), vals.as<uint32_t>(), ff.as<float>(), ff.as<float>(), cnt.as<int>(), cap};
     // the lapd sample slot aliases ff; nothing reads it here
-    pb.lap = nullptr;
-    DevBuf lapdummy;
     lapdummy.ensure(cap * 4);
     pb.lap = lapdummy.as<float>();
     launch_peakfind(Launch{s, &ctx->sync.launches}, dd, nullptr, dm, n1, n2, n3, n1, (int64_t)n1 * n2, nbuff, fcrit,
@@ -197,7 +216,10 @@ static int32_t analyse_peaks_impl(ppb_ctx* ctx, const float* delta, const float*
     std::shared_lock<std::shared_mutex> rl(ctx->sh.mu);
     ShellTable& shells = ctx->shell_table(nhunt, s);
     // fields -> contiguous device staging -> packed gather records
-    DevBuf st_delta, st_psi, st_psi2, st_lapd, aos, d_ipp, d_lin, d_Rf, d_ir2in, d_ir2, d_Z, d_fc, d_out, d_lim;
+    StubCall call(ctx->sync);
+    DevBuf &st_delta = call[0], &st_psi = call[1], &st_psi2 = call[2], &st_lapd = call[3], &aos = call[4],
+           &d_ipp = call[5], &d_lin = call[6], &d_Rf = call[7], &d_ir2in = call[8], &d_ir2 = call[9], &d_Z = call[10],
+           &d_fc = call[11], &d_out = call[12], &d_lim = call[13];
     st_psi.ensure(3 * N * 4);
     auto put = [&](DevBuf& b, size_t off, const float* src) {
       PPB_CUDA(cudaMemcpyAsync((char*)b.p + off, src, N * 4, cudaMemcpyDefault, s));
@@ -307,8 +329,11 @@ int32_t ppb_analyse_peaks_multirf(ppb_ctx* ctx, const float* delta, const float*
     const int64_t N = (int64_t)n * n * n;
     std::shared_lock<std::shared_mutex> rl(ctx->sh.mu);
     ShellTable& shells = ctx->shell_table(nhunt, s);
-    DevBuf st_delta, st_psi, st_psi2, st_lapd, aos, d_pi, d_pj, d_pk, d_Zpp, d_fpp, d_mask, d_out;
-    DevBuf p_lin, p_Rf, p_ir2, p_np, p_Z, p_fc, p_skip;
+    StubCall call(ctx->sync);
+    DevBuf &st_delta = call[0], &st_psi = call[1], &st_psi2 = call[2], &st_lapd = call[3], &aos = call[4],
+           &d_pi = call[5], &d_pj = call[6], &d_pk = call[7], &d_Zpp = call[8], &d_fpp = call[9], &d_mask = call[10],
+           &d_out = call[11], &p_lin = call[12], &p_Rf = call[13], &p_ir2 = call[14], &p_np = call[15],
+           &p_Z = call[16], &p_fc = call[17], &p_skip = call[18];
     st_psi.ensure(3 * N * 4);
     auto put = [&](DevBuf& b, size_t off, const float* src) {
       PPB_CUDA(cudaMemcpyAsync((char*)b.p + off, src, N * 4, cudaMemcpyDefault, s));
