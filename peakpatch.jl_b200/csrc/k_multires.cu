@@ -413,18 +413,9 @@ __device__ __forceinline__ void tri_sum(const float* coarse, const int4& ix, con
 #pragma unroll
         for (int u = 0; u < KZ; u++) {
           const float w3 = __fmul_rn(wij[b][c], comp(wz[u], a));
-          if constexpr (NF % 2 == 0) {   // two fields per instruction, each rounded as the scalar form
+          // scalar intrinsics: the packed pair __fmul2_rn, __fadd2_rn is compiled into one fused operation
 #pragma unroll
-            for (int f = 0; f < NF; f += 2) {
-              const float2 p = __fmul2_rn(make_float2(w3, w3), make_float2(v[f], v[f + 1]));
-              const float2 s = __fadd2_rn(make_float2(val[u][f], val[u][f + 1]), p);
-              val[u][f] = s.x;
-              val[u][f + 1] = s.y;
-            }
-          } else {
-#pragma unroll
-            for (int f = 0; f < NF; f++) val[u][f] = __fadd_rn(val[u][f], __fmul_rn(w3, v[f]));
-          }
+          for (int f = 0; f < NF; f++) val[u][f] = __fadd_rn(val[u][f], __fmul_rn(w3, v[f]));
         }
       }
     }
