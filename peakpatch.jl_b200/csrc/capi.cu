@@ -447,7 +447,7 @@ TuneEntry ppb_ctx::tune_shells(Slot& sl, const ShellArgs& b0, bool comp, bool ad
   // collapse: the size heuristic's width in list order unless another
   // (width, order) is at least 3 % faster
   const int wd = shell_collapse_width(b.npk, nsm, sl.walk_per_peak);
-  const int di = wd == 4 ? 2 : wd - 1;
+  const int di = wd >= 4 ? 2 : wd - 1;   // a batch that is tuned is too large for a warp per peak
   int ci = di, co = 0;
   for (int o = 0; o < 2; o++)
     for (int c = 0; c < 4; c++) {

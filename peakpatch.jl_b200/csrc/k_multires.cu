@@ -425,7 +425,7 @@ __device__ __forceinline__ void tri_sum(const float* coarse, const int4& ix, con
 // A thread owns kTriZ cells of consecutive lk: they almost always lie in the
 // same coarse cell (a block of N / M fine cells), and the coarse values are
 // then loaded once for all (the loads bound the kernel: one cell per thread
-// took 0.35 ms for a 192^3 tile of four fields, this takes 0.18).  The planes of a
+// took 0.35 ms for a 192^3 tile of four fields, this takes 0.22).  The planes of a
 // block's cells are the same for all its threads.
 constexpr int kTriZ = 4;
 template <int NF>

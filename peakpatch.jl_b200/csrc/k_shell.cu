@@ -1107,9 +1107,11 @@ __device__ __forceinline__ void write_no_collapse(double* o) {
 // Phases 6-7 of a collapsed peak (RadialShell.jl:707-790) and its result
 // row: m0 is the shell above the first collapsing step, last / prev the
 // kernel_strain values of that step and of the step before it (zvir1p /
-// zvir1 their zvir), lastFh the trace at the collapsing step.
+// zvir1 their zvir), lastFh the trace at the collapsing step; sums: phase 7's
+// sums, or null to form them here.
 __device__ void collapse_finish(const ShellArgs& a, const Rows& R, double ZZon, int m0, double zvir1, double zvir1p,
-                                const KS& prev, const KS& last, double lastFh, const double* grf, double* out) {
+                                const KS& prev, const KS& last, double lastFh, const double* grf, double* out,
+                                const double* sums = nullptr) {
   const double* __restrict__ rad = a.rad;
   // Phase 6: collapse radius (RadialShell.jl:707-754)
   const double dZvir = zvir1p - zvir1;
@@ -1169,7 +1171,12 @@ __device__ void collapse_finish(const ShellArgs& a, const Rows& R, double ZZon, 
   double sb[6] = {0, 0, 0, 0, 0, 0};
   long long nS = 0;
   double srb = 0.0;
-  for (int m1 = 1; m1 <= m0 - 1; m1++) {
+  if (sums) {   // formed by the warp (coop_sums)
+#pragma unroll
+    for (int q = 0; q < 6; q++) sb[q] = sums[q];
+    nS = (long long)sums[6];
+    srb = sums[7];
+  } else for (int m1 = 1; m1 <= m0 - 1; m1++) {
     const double nn = R.get(R_N, m1);
     if (nn > 0) {
 #pragma unroll
@@ -1297,7 +1304,7 @@ __device__ __forceinline__ KS shfl_ks(const KS& k, int src, unsigned mask) {
   return r;
 }
 
-// QT threads per peak (lanes qbase .. qbase+QT-1, QT = 2 or 4): the inward
+// QT threads per peak (lanes qbase .. qbase+QT-1, QT = 2): the inward
 // walk evaluates QT consecutive steps per round, thread q taking step
 // base + q (mp = m0 - step; step 0 is the m0 step, whose zvir is forced to
 // -1), and the group takes the first step that collapses; the step before it
@@ -1388,6 +1395,245 @@ __device__ void collapse_group(const ShellArgs& a, int64_t p, int q, int qbase, 
   collapse_finish(a, R, ZZon, m0, zvir1, zvir1p, prev, last, lastFh, grf, out);
 }
 
+// ---------------------------------------------------------------------------
+// Cooperative row sums.  A lane that sums a window of its peak's rows alone
+// reads 16 bytes of a row per load while its neighbours read other rows: one
+// cache line looked up per lane, which bounded the collapse kernels.  Here
+// the warp's tasks (at most one per lane) are taken four at a time, eight
+// lanes per task, one value of the row per lane, so that a row's values are
+// one or two lines for all of them.  Each value is summed by one lane in
+// shell order: the sums are those of a lane working alone.
+// ---------------------------------------------------------------------------
+// the task of a subgroup of eight lanes in round it of `mask`'s tasks, -1: none
+__device__ __forceinline__ int coop_task(unsigned mask, int it, int sub) {
+  for (int s = 4 * it + sub; s > 0 && mask; s--) mask &= mask - 1;
+  return mask ? __ffs(mask) - 1 : -1;
+}
+
+// kernel_strain's six values from `first` on (R_Q: the strain E, weights -wt
+// / 2; R_G: the gradients g and gf) for the lanes with act: centre shell mp
+// over the shells [lo, hi] of the rows at pool row `off` with rows up to
+// mdone.  Called by whole warps.
+template <bool STRAIN>
+__device__ __forceinline__ void coop_strain(const ShellArgs& a, bool act, long long off, int mdone, int mp, int lo,
+                                            int hi, double wRnor, double aRnor, double (&v)[6]) {
+  const int lane = threadIdx.x & 31, sub = lane >> 3, c = lane & 7;
+  const unsigned mask = __ballot_sync(FULL, act);
+  int wi = 0;   // weight of shell m1: wts[wi + m1], or w1[m1]
+  double scale = 0.0;
+  if (act) {
+    if (mp > 1) {
+      const int wl = __ldg(a.win_lo + mp), wh = __ldg(a.win_hi + mp);
+      lo = max(lo, wl);
+      hi = min(hi, wh);
+      wi = __ldg(a.win_off + mp) - wl;
+      scale = wRnor / __ldg(a.rad + mp);
+    } else {
+      scale = aRnor;
+    }
+    if (hi > mdone) {                 // never taken when the truncation rule holds
+      atomicAdd(a.counters + CNT_GUARD, 1ull);
+      hi = mdone;
+    }
+  }
+  const int ntask = __popc(mask), rank = __popc(mask & ((1u << lane) - 1u));
+  for (int it = 0; 4 * it < ntask; it++) {
+    const int t = coop_task(mask, it, sub), src = t < 0 ? 0 : t;
+    const int tlo = __shfl_sync(FULL, lo, src), thi = __shfl_sync(FULL, hi, src), tmp = __shfl_sync(FULL, mp, src),
+              twi = __shfl_sync(FULL, wi, src);
+    const long long toff = __shfl_sync(FULL, off, src);
+    double acc = 0.0;
+    if (t >= 0 && c < 6) {
+      const double* w = tmp > 1 ? a.wts + twi : a.w1;
+      const double* row = a.pool + toff * ROW + (STRAIN ? R_Q : R_G) + c;
+      auto add = [&](double wt, double x) {
+        if (c == 0 && tmp == 1 && isnan(wt)) atomicAdd(a.counters + CNT_AKK, 1ull);
+        acc = STRAIN ? fma(-(0.5 * wt), x, acc) : fma(wt, x, acc);
+      };
+      int m1 = tlo;
+      for (; m1 + 7 <= thi; m1 += 8) {   // eight rows in flight
+        double wt[8], x[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+          wt[u] = __ldg(w + m1 + u);
+          x[u] = row[(int64_t)(m1 + u) * ROW];
+        }
+#pragma unroll
+        for (int u = 0; u < 8; u++) add(wt[u], x[u]);
+      }
+      for (; m1 <= thi; m1++) add(__ldg(w + m1), row[(int64_t)m1 * ROW]);
+    }
+    const bool mine = act && (rank >> 2) == it;
+#pragma unroll
+    for (int q = 0; q < 6; q++) {
+      const double x = __shfl_sync(FULL, acc, (rank & 3) * 8 + q);
+      if (mine) v[q] = x * scale;
+    }
+  }
+}
+
+// Phase 7's sums over the shells 1 .. m0 - 1 (RadialShell.jl:758-790) for the
+// lanes with act: Sbar and Sbar2 over shells with cells, the cells, and the
+// Srb integral, each in shell order
+__device__ __forceinline__ void coop_sums(const ShellArgs& a, bool act, long long off, int mdone, int m0,
+                                          double (&v)[8]) {
+  const int lane = threadIdx.x & 31, sub = lane >> 3, c = lane & 7;
+  const unsigned mask = __ballot_sync(FULL, act);
+  int hi = m0 - 1;
+  if (act && hi > mdone) {   // never taken when the truncation rule holds
+    atomicAdd(a.counters + CNT_GUARD, 1ull);
+    hi = mdone;
+  }
+  const int ntask = __popc(mask), rank = __popc(mask & ((1u << lane) - 1u));
+  for (int it = 0; 4 * it < ntask; it++) {
+    const int t = coop_task(mask, it, sub), src = t < 0 ? 0 : t;
+    const int thi = __shfl_sync(FULL, hi, src);
+    const long long toff = __shfl_sync(FULL, off, src);
+    double acc = 0.0;
+    if (t >= 0) {
+      const double* rows = a.pool + toff * ROW;
+      const int col = c < 6 ? R_S + c : c == 6 ? R_N : R_FBAR;   // R_S2 = R_S + 3
+      double fp = 0.0, r5p = 0.0;
+      auto add = [&](int m1, double x, double nn, double r5) {
+        if (c == 7) {
+          if (m1 >= 2) acc += 0.5 * (fp + x) * (r5 - r5p);
+          fp = x;
+          r5p = m1 >= 2 ? r5 : 0.0;
+        } else if (nn > 0) {
+          acc += c == 6 ? (double)(long long)nn : x;
+        }
+      };
+      int m1 = 1;
+      for (; m1 + 3 <= thi; m1 += 4) {
+        double x[4], nn[4], r5[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+          x[u] = rows[(int64_t)(m1 + u) * ROW + col];
+          nn[u] = rows[(int64_t)(m1 + u) * ROW + R_N];
+          r5[u] = __ldg(a.rad5 + m1 + u);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; u++) add(m1 + u, x[u], nn[u], r5[u]);
+      }
+      for (; m1 <= thi; m1++)
+        add(m1, rows[(int64_t)m1 * ROW + col], rows[(int64_t)m1 * ROW + R_N], __ldg(a.rad5 + m1));
+    }
+    const bool mine = act && (rank >> 2) == it;
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+      const double x = __shfl_sync(FULL, acc, (rank & 3) * 8 + q);
+      if (mine) v[q] = x;
+    }
+  }
+}
+
+// QT threads per peak (QT = 4 or 32; 32 / QT peaks per warp): the inward walk
+// (RadialShell.jl:566-699) evaluates up to QT consecutive steps per round, lane q of a peak taking step base + q (mp = m0 - step; step 0 is the
+// m0 step, whose zvir is forced to -1), and the peak takes the first step
+// that collapses; the step before it comes from the lane to its left or, for
+// q = 0, from the previous round's last step.  Only the strain is needed to
+// walk; the gradients are formed for the two steps a collapse interpolates
+// between.  The row sums run on the whole warp (coop_strain), so every lane
+// stays in the loop until the warp's last walk ends.  With 32 lanes the first
+// round takes kFirst steps, since most walks of a single-redshift tile end
+// there.
+// Measured against four lanes that each read their own window: 13,600 peaks
+// of a 128^3 tile 0.44 -> 0.28 ms, four lightcone tiles of 192^3 5.3 -> 3.9;
+// one and two lanes per peak keep their own windows, being faster so on full
+// batches (384^3, two lanes 3.15 ms; with the shared sums 3.55) and on the
+// few rows of small shell lists.
+constexpr int kFirst = 8;
+template <int QT>
+__device__ void collapse_lanes(const ShellArgs& a, bool valid, int64_t p) {
+  const int lane = threadIdx.x & 31, q = lane & (QT - 1), qbase = lane & ~(QT - 1);
+  const unsigned qbits = QT == 32 ? FULL : (1u << QT) - 1u;
+  double* out = a.out + p * RES_N;
+  PeakHdr h{};
+  if (valid) h = a.hdr[p];
+  const bool run = valid && h.status == HS_OK;
+  if (valid && !run && q == 0) write_no_collapse(out);
+  const double* __restrict__ rad = a.rad;
+  const Rows R{a.pool + h.off * ROW, h.mdone, a.counters};
+  const double alatt = a.alatt, anor = 1.0;
+  const double aRnor = 3.0 * anor / alatt, wnor = anor / (4.0 * 3.141592653589793), wRnor = 3.0 * wnor / alatt;
+  double ZZon = 0.0;
+  int m = 1, hi1 = 1;
+  int4 gq = make_int4(1, 1, 1, 1);   // (m0_init, mrf, mlow_rf, mupp_rf)
+  if (run) {
+    ZZon = a.pk.ZZon[p];
+    m = a.mlim[p];
+    gq = a.geo[2 * p];
+    hi1 = last_lt(rad, 2, m, 2.0);   // at mp = 1 the running window is [2, last shell with rad < 2]
+  }
+  const int m0o = h.m0;
+  int m0 = m0o;
+  double E[6] = {0, 0, 0, 0, 0, 0}, lastE[6], prevE[6], carry[6] = {0, 0, 0, 0, 0, 0};
+  double zcarry = -1.0, zvir1 = -1.0, zvir1p = -1.0, lastFh = 0.0;
+  bool walking = run, collapsed = false;
+  for (int base = 0, cnt = QT == 32 ? kFirst : QT; __any_sync(FULL, walking); base += cnt, cnt = QT) {
+    const int st = base + q, mp = m0o - st;
+    const bool act = walking && q < cnt && mp >= 1;
+    coop_strain<true>(a, act, h.off, h.mdone, mp, 2, mp > 1 ? m : hi1, wRnor, aRnor, E);
+    double zv = -1.0, Fh = 0.0;
+    if (act && st >= 1) {
+      double ev, pv;
+      ev_pv(E, &Fh, &ev, &pv);
+      zv = zvir_of(a.tab, R.get(R_FBAR, mp), ev, pv);
+    }
+    const unsigned hits = (__ballot_sync(FULL, act && st >= 1 && zv >= ZZon) >> qbase) & qbits;
+    const int qs = hits ? __ffs(hits) - 1 : 0, ql = qs > 0 ? qs - 1 : 0;
+    const bool now = walking && hits != 0;
+    const double Fhs = __shfl_sync(FULL, Fh, qbase + qs), zs = __shfl_sync(FULL, zv, qbase + qs),
+                 zl = __shfl_sync(FULL, zv, qbase + ql), zc = __shfl_sync(FULL, zv, qbase + cnt - 1);
+#pragma unroll
+    for (int i = 0; i < 6; i++) {
+      const double es = __shfl_sync(FULL, E[i], qbase + qs), el = __shfl_sync(FULL, E[i], qbase + ql),
+                   ec = __shfl_sync(FULL, E[i], qbase + cnt - 1);
+      if (now) {
+        lastE[i] = es;
+        prevE[i] = qs > 0 ? el : carry[i];
+      }
+      carry[i] = ec;
+    }
+    if (now) {
+      lastFh = Fhs;
+      zvir1p = zs;
+      zvir1 = qs > 0 ? zl : zcarry;
+      m0 = m0o - (base + qs) + 1;
+      collapsed = true;
+      walking = false;
+    }
+    zcarry = zc;
+    if (m0o - (base + cnt - 1) <= 1) walking = false;   // walked down to mp = 1
+  }
+  if (run && q == 0) {   // the walk's own steps, not those evaluated past its end
+    atomicAdd(a.counters + CNT_WALK, (unsigned long long)(collapsed ? m0o - m0 + 2 : m0o));
+    if (!collapsed) {
+      atomicAdd(a.counters + CNT_NOCOLL, 1ull);
+      write_no_collapse(out);
+    }
+  }
+  // the collapsed peaks: gradients of the collapsing step and of the one
+  // before it, phase 3's gradient at the filter scale, phase 7's sums
+  const bool fin = collapsed && q == 0;
+  if (__ballot_sync(FULL, fin) == 0) return;
+  KS last, prev;
+  double g[6], grf[6], sums[8];
+  coop_strain<false>(a, fin, h.off, h.mdone, m0 - 1, 2, m0 - 1 > 1 ? m : hi1, wRnor, aRnor, g);
+#pragma unroll
+  for (int L = 0; L < 3; L++) { last.g[L] = g[L]; last.gf[L] = g[3 + L]; }
+  coop_strain<false>(a, fin, h.off, h.mdone, m0, 2, m0 > 1 ? m : hi1, wRnor, aRnor, g);
+#pragma unroll
+  for (int L = 0; L < 3; L++) { prev.g[L] = g[L]; prev.gf[L] = g[3 + L]; }
+  coop_strain<false>(a, fin, h.off, h.mdone, gq.y, gq.z, gq.w, wRnor, aRnor, grf);
+  coop_sums(a, fin, h.off, h.mdone, m0, sums);
+  if (fin) {
+#pragma unroll
+    for (int i = 0; i < 6; i++) { last.E[i] = lastE[i]; prev.E[i] = prevE[i]; }
+    collapse_finish(a, R, ZZon, m0, zvir1, zvir1p, prev, last, lastFh, grf, out, sums);
+  }
+}
+
 // the peak of collapse slot i: i itself, or its place in the collapse order
 __device__ __forceinline__ int64_t collapse_peak(const ShellArgs& a, int64_t i) {
   return a.corder ? (int64_t)__ldg(a.corder + i) : i;
@@ -1404,6 +1650,13 @@ __global__ void __launch_bounds__(128) collapse_kernel(ShellArgs a) {
   const int64_t i = t / QT;
   const int lane = threadIdx.x & 31, q = lane & (QT - 1), qbase = lane & ~(QT - 1);
   if (i < a.npk) collapse_group<QT>(a, collapse_peak(a, i), q, qbase, ((1u << QT) - 1u) << qbase);
+}
+
+template <int QT>
+__global__ void __launch_bounds__(128) collapse_lanes_kernel(ShellArgs a) {
+  const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / QT;
+  const bool valid = i < a.npk;   // lanes past the batch stay for the warp's row sums
+  collapse_lanes<QT>(a, valid, collapse_peak(a, valid ? i : 0));
 }
 
 // collapse order key (thread per peak): peaks that reach the walk by
@@ -1763,7 +2016,8 @@ int shell_collapseq_blocks(int nsm) {
 }
 
 int shell_collapse_width(int64_t npk, int nsm, double walk_steps_per_peak) {
-  // 4 threads per peak while 4 per peak still fit about 24 warps per SM or
+  // a warp per peak for small batches (7,002 peaks: 0.41 ms with four threads
+  // each reading its own window, 0.28 so), 4 threads per peak while 4 per peak still fit about 24 warps per SM or
   // when walks are long (more than 8 steps per peak in the previous batch:
   // the lightcone), else 2 or 1 (the device is full and the latency hidden)
   const int64_t full = (int64_t)nsm * 24 * 32;
@@ -1782,13 +2036,16 @@ void launch_shell_collapse(Launch L, const ShellArgs& a, int nsm, double walk_st
     return;
   }
   if (w != 1 && w != 2 && w != 4) w = shell_collapse_width(a.npk, nsm, walk_steps_per_peak);
-  const int lg = w == 4 ? 2 : w - 1;
+  const int lg = w == 32 ? 5 : w == 4 ? 2 : w - 1;
   const int64_t blocks = ((a.npk << lg) + 127) / 128;
+constexpr int64_t kWarpPeaks = 12000;   // 81 warps per SM
   if (blocks == 0) return;
-  if (w == 4) collapse_kernel<4><<<(unsigned)blocks, 128, 0, L.s>>>(a);
+  if (w == 32) collapse_lanes_kernel<32><<<(unsigned)blocks, 128, 0, L.s>>>(a);
+  else if (w == 4) collapse_lanes_kernel<4><<<(unsigned)blocks, 128, 0, L.s>>>(a);
   else if (w == 2) collapse_kernel<2><<<(unsigned)blocks, 128, 0, L.s>>>(a);
   else collapse1_kernel<<<(unsigned)blocks, 128, 0, L.s>>>(a);
   PPB_LAUNCHED(*L.count);
+  if (npk <= kWarpPeaks) return 32;
 }
 
 void launch_shell_zhalf(Launch L, const ShellArgs& a) {
