@@ -110,13 +110,20 @@ void build_shell_table(ShellTable& st, int nhunt) {
   // small shells), so that the lanes split the cells of each shell
   int total = 0;
   for (int m = 2; m <= mmax; m++) total += st.shell_count[m - 1];
+  // and smaller in the first groups, where most peaks of a tile stop (a group
+  // is gathered whole, so its size is the truncation's grain): with
+  // kFirstChunk cells in the first kFirstGroups groups the 384^3 tile visits
+  // 6.9e8 cells instead of 8.2e8 (8.20 -> 7.61 ms), while whole spheres of
+  // thousands of cells keep the larger chunks (200,000 peaks to 24 cells:
+  // 5.32 ms with 24 throughout, 6.11 with 16, 5.36 so)
   const int csize = std::min(kChunkCells, std::max(4, 4 * ((total + 127) / 128)));
+  const int cfirst = std::min(csize, kFirstChunk);
   for (int m = 2; m <= mmax; m++) {
     const int cnt = st.shell_count[m - 1], s0 = st.shell_start[m - 1];
-    int nck = (cnt + csize - 1) / csize;
-    if (nck > 32) nck = 32;
-    if (nck < 1) nck = 1;
+    auto chunks = [&](int cs) { return std::min(32, std::max(1, (cnt + cs - 1) / cs)); };
+    int nck = chunks((int)st.grp_a.size() <= kFirstGroups ? cfirst : csize);
     if (in_group + nck > 32 || st.grp_a.empty()) {   // open a new group
+      nck = chunks((int)st.grp_a.size() < kFirstGroups ? cfirst : csize);
       if (!st.grp_a.empty()) st.grp_b.back() = m - 1;
       st.grp_a.push_back(m);
       st.grp_b.push_back(m);

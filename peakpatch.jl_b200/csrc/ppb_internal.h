@@ -78,6 +78,7 @@ struct DevBuf {
 // geometry of the sorted shell-cell list (precompute_shells)
 // ---------------------------------------------------------------------------
 constexpr int kChunkCells = 24;   // gather chunk size (cells per lane per group; smaller for short lists)
+constexpr int kFirstChunk = 16, kFirstGroups = 2;   // and in the first groups
 
 struct ShellTable {
   int nhunt = -1;
