@@ -403,6 +403,19 @@ TuneEntry ppb_ctx::tune_shells(Slot& sl, const ShellArgs& b0, bool comp, bool ad
     for (int o = 0; o < 2; o++) {   // list order, then by descending crossing shell
       for (int c = 0; c < 4; c++) {
         PPB_CUDA(cudaEventRecord(ev[0], s));
+      if (round == 0 && c == 0) {
+        // rows past the pool's end: most peaks are marked overflowed, and the
+        // times of what follows would say nothing
+        unsigned long long used = 0;
+        PPB_CUDA(cudaMemcpyAsync(&used, b.pool_ctr, sizeof(used), cudaMemcpyDeviceToHost, s));
+        PPB_CUDA(cudaStreamSynchronize(s));
+        if ((int64_t)used > b.pool_cap) {
+          PPB_CUDA(cudaMemcpyAsync(sl.counters.p, sl.tune_save.p, 16 * 8, cudaMemcpyDeviceToDevice, s));
+          PPB_CUDA(cudaMemsetAsync(sl.ctl.p, 0, kCtlBytes, s));
+          te.npk = 0;
+          return te;
+        }
+      }
         collapse_order(sl, b, o == 1);
         launch_shell_collapse(L, b, nsm, sl.walk_per_peak, widths[c]);
         PPB_CUDA(cudaEventRecord(ev[1], s));
@@ -507,13 +520,16 @@ void ppb_ctx::run_shells(Slot& sl, ShellArgs& a, bool comp, bool adaptive, Shell
   if (rpp <= 0.0) rpp = adaptive ? 64.0 : (double)(a.mmax + 1);
   // pool budget: half of the free memory (with the pool's own), at most 32 GB;
   // the free-memory query runs only when the pool would have to grow
-  int64_t budget_rows = (int64_t)(sl.pool.bytes / row_bytes);
-  if ((double)a.npk * rpp * 1.25 + 4096 > (double)budget_rows) {
+  int64_t budget_rows = 0;
+  auto set_budget = [&](double peaks) {
+    budget_rows = (int64_t)(sl.pool.bytes / row_bytes);
+    if (peaks * rpp * 1.25 + 4096 <= (double)budget_rows) return;
     size_t fr = 0, tot = 0;
     PPB_CUDA(cudaMemGetInfo(&fr, &tot));
     budget_rows = std::max<int64_t>(
         1 << 16, (int64_t)(std::min<size_t>((size_t)32 << 30, (fr + sl.pool.bytes) / 2) / row_bytes));
-  }
+  };
+  set_budget((double)a.npk);
   ShellStats s{};
   unsigned long long before[16] = {}, c[16] = {};
   // autotuned order brick and collapse width for this kind of batch
@@ -577,13 +593,15 @@ void ppb_ctx::run_shells(Slot& sl, ShellArgs& a, bool comp, bool adaptive, Shell
     if (tune_now) {
       if (first && pre) pre();   // the tuning pass reads what `pre` writes
       te = tune_shells(sl, b, comp, adaptive, gblocks, rmap);
-      {
+      if (te.npk > 0) {
         std::lock_guard<std::mutex> lk(sh.cache_mu);
         sh.tune[tkey] = te;
       }
-      tune_now = false;
     }
     const int fb = sh.force_brick.load(), fc = sh.force_collapse.load();
+        tune_now = false;
+      } else {   // the pool was too small: the run below finds its size, then the tuning is repeated
+        te = TuneEntry();
     const int fo = sh.collapse_order.load();
     const bool corder_on = fo == 1 || (fo == -1 && te.collapse_order);
     if (sh.gather_tex.load() == -1 && !te.gather_tex) b.rec_tex = 0;
@@ -622,6 +640,7 @@ void ppb_ctx::run_shells(Slot& sl, ShellArgs& a, bool comp, bool adaptive, Shell
     }
     float k[4];
     for (int e = 0; e < 4; e++) PPB_CUDA(cudaEventElapsedTime(&k[e], sl.shell_ev[e], sl.shell_ev[e + 1]));
+      set_budget((double)(a.npk - p0));
     for (int e = 0; e < 4; e++) s.kms[e] += k[e];
     s.ms += k[0] + k[1] + k[2] + k[3];
     s.pool_rows += used;
@@ -635,6 +654,10 @@ void ppb_ctx::run_shells(Slot& sl, ShellArgs& a, bool comp, bool adaptive, Shell
   for (int i = 0; i < 5; i++) s.dump[i] = c[1 + i];
   s.guard = c[6];
   s.akk = c[7];
+  // the next call's estimate: the rows per peak of the whole call (the last
+  // batch's alone would be the small radii's, and the first batch of the next
+  // call would overflow the pool and run twice)
+  if (s.batches > 1) rpp = std::max(1.0, (double)s.pool_rows / (double)a.npk);
   for (int i = 0; i < 16; i++) s.raw[i] = c[i];
   sl.last_shell = s;
   if (st) *st = s;
