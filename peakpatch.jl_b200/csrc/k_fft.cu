@@ -72,7 +72,7 @@ struct ColOut {
 struct ColArgs {
   ColOut o[kTwinGroup];
   const float2* tw;
-  const float2* win;      // kind 3: (W, W_3) by q, wstride apart per output
+  const float* win;       // kind 3: W_3 by q, wstride apart per output
   int64_t wstride;
   int nout;
   int kind;               // transfer applied as the input is read (z passes): 0 none, 1 ps / q, 2 q ps, 3 W_3(q) ps
@@ -118,7 +118,7 @@ __global__ void __launch_bounds__(kColW* kLanes<N>, kColBlocks<N>) col_kernel(co
         float s;
         if (a.kind == 1) s = q ? __fdividef(a.ps, (float)q) : 0.f;
         else if (a.kind == 2) s = (float)q * a.ps;
-        else s = __ldg(a.win + o * a.wstride + (live ? q : 0)).y * a.ps;
+        else s = __ldg(a.win + o * a.wstride + (live ? q : 0)) * a.ps;
         if (znp || (a.zero_nyq && e == N / 2)) s = 0.f;
         v[j].x *= s;
         v[j].y *= s;
@@ -530,7 +530,7 @@ void lpt2_n(Launch L, const float2* dk, const float* delta, float2* const* w, co
 // kind 3 with one window table (wstride float2 apart) and frequency limit each
 template <int N>
 void zy_n(Launch L, const float2* dk, float2* const* w, int cnt, const float2* tw, int kind, float ps,
-          const float2* win, int64_t wstride, bool zero_nyq, const int* flim) {
+          const float* win, int64_t wstride, bool zero_nyq, const int* flim) {
   int fmax = 0;
   for (int i = 0; i < cnt; i++) fmax = flim[i] > fmax ? flim[i] : fmax;
   ColArgs z = col_args(tw, N, fmax);
@@ -559,7 +559,8 @@ template <int N> void rows_n(Launch L, const float2* w, float* out, const float2
 }
 
 #define PPB_FFT_SIZES(X) \
-  X(4) X(5) X(6) X(7) X(8) X(9) X(10) X(11) X(12) X(14) X(15) X(16) X(18) X(20) X(21) X(22) X(24) X(28) X(32)
+  X(4) X(5) X(6) X(7) X(8) X(9) X(10) X(11) X(12) X(13) X(14) X(15) X(16) X(17) X(18) X(19) X(20) X(21) X(22) \
+  X(23) X(24) X(28) X(32)
 
 }  // namespace
 
@@ -623,7 +624,7 @@ void launch_twin_zy(Launch L, const float2* dk, float2* const* w, int cnt, const
   switch (n / 16) {
 #define X(m) \
   case m: \
-    zy_n<16 * m>(L, dk, w, cnt, tw, 3, ps, reinterpret_cast<const float2*>(tab), tab_stride / 2, false, flim); \
+    zy_n<16 * m>(L, dk, w, cnt, tw, 3, ps, tab, tab_stride, false, flim); \
     break;
     PPB_FFT_SIZES(X)
 #undef X

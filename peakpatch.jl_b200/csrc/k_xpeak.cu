@@ -378,7 +378,7 @@ __global__ void __launch_bounds__(256) window_t_kernel(const float2* __restrict_
       const int ky = ky0 + ty + 8 * u;
       const int fy = ky <= nyq ? ky : ky - n;
       d[u] = __ldg(dk + ((int64_t)kz * n + ky) * nh + kx);
-      w[u] = __ldg(tab + 2 * (kx * kx + fy * fy + fz * fz));
+      w[u] = __ldg(tab + (kx * kx + fy * fy + fz * fz));
     }
 #pragma unroll
     for (int u = 0; u < 4; u++)

@@ -68,7 +68,7 @@ template <int SIGN> __device__ __forceinline__ float2 rot(float2 a, float c, flo
   return make_float2(fmaf(a.x, c, -a.y * t), fmaf(a.x, t, a.y * c));
 }
 
-constexpr int first_factor(int R) {   // 4 before 2, then 3, 5, 7, 11
+constexpr int first_factor(int R) {   // 4 before 2, then 3, 5, 7, else a prime (R < 64)
   return R % 4 == 0 && R != 4 ? 4 : R % 2 == 0 && R != 2 && R != 4 ? 2 : R % 3 == 0 ? 3 : R % 5 == 0 ? 5 : R % 7 == 0 ? 7 : R;
 }
 

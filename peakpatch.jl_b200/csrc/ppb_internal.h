@@ -275,9 +275,9 @@ void launch_phi(Launch L, const float2* dk, float2* out, int n, double boxsize, 
 void launch_src2(Launch L, const float* phi, float* out, int64_t N);
 void launch_lpt2(Launch L, const float2* s2k, float2* out, int n, double boxsize, double post_scale);
 void launch_lapd(Launch L, const float2* dk, float2* out, int n, double boxsize, float post_scale);
-// window tables: per filter f, window_table_size(n) float pairs (W_wsmooth,
-// the k^2-weighted Gaussian of the Laplacian diagnostic) by integer |k|^2 at
-// tab + f * 2 * window_table_size(n); Rf is a device array of nfilt radii
+// window tables: per filter f, window_table_size(n) floats W_wsmooth, then as
+// many of the k^2-weighted Gaussian of the Laplacian diagnostic, by integer
+// |k|^2 at tab + f * 2 * window_table_size(n); Rf: device array of nfilt radii
 int window_table_size(int n);
 void launch_window_tables(Launch L, float* tab, int n, double boxsize, const double* Rf, int nfilt, int wsmooth,
                           bool want_lap);
@@ -331,7 +331,7 @@ void launch_xpeak(Launch L, const float2* ds, const float2* tw, uint8_t* mask, i
                   unsigned long long keyhi, PeakBuf pb);
 
 // transforms with fused k-space and real-space work (k_fft.cu), for grid
-// sizes 16 M with M up to 32 of factors 2, 3, 5, 7, 11 (fft_supported).  Rows
+// sizes 16 M, M = 4 .. 24, 28 or 32 (fft_supported).  Rows
 // of the work arrays are fft_pitch(n) float2; tw[k] = exp(2 pi i k / n).
 bool fft_supported(int n);
 int fft_pitch(int n);
@@ -348,7 +348,7 @@ void launch_lpt2_fused(Launch L, const float2* dk, const float* delta, float2* c
 void launch_laplacian_fused(Launch L, const float2* dk, float2* w, const float2* tw, float* out, int n, float scale,
                             bool zero_nyq);
 // z and y transforms of the k^2-weighted twins of `cnt` <= kTwinGroup
-// consecutive filters (window tables tab_stride floats apart) into w[i]
+// consecutive filters (W_3 tables tab_stride floats apart) into w[i]
 // [z][y][kx], frequencies up to flim[i] = twin_flim(n, box, Rf); then their
 // values at the peaks of slots *first .. count - 1, whose keys hold the
 // filter (from f0) and the cell of an n1 x n2 window (starting at

@@ -647,7 +647,7 @@ int64_t peaks_phase(Run& r, TileRes& T, int n, double box, const std::vector<Win
           const int f0 = f / group * group, cnt = f - f0 + 1;
           int flim[kTwinGroup];
           for (int i = 0; i < cnt; i++) flim[i] = twin_flim(n, box, r.Rf[f0 + i]);
-          launch_twin_zy(L, dkp, tw_w, cnt, T.xtw.as<float2>(), n, T.wtab.as<float>() + (size_t)f0 * 2 * qn, 2 * qn,
+          launch_twin_zy(L, dkp, tw_w, cnt, T.xtw.as<float2>(), n, T.wtab.as<float>() + (size_t)f0 * 2 * qn + qn, 2 * qn,
                          (float)inv_n3, flim);
           launch_twin_rows(L, tw_w, cnt, T.xtw.as<float2>(), n, flim, nm, nm, r.fbits, f0,
                            wins.size() > 1 ? r.sl->woff.as<int64_t>() : nullptr, first, pb);

@@ -11,9 +11,10 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
-# every factor of the register transforms (2, 3, 5, 7, 11), the smallest and
+# every factor of the register transforms, the smallest and
 # largest size, sizes with more and with fewer threads than 16 per column
-SIZES = [64, 80, 96, 112, 128, 144, 160, 176, 192, 224, 240, 256, 288, 320, 336, 352, 384, 448, 512]
+SIZES = [64, 80, 96, 112, 128, 144, 160, 176, 192, 208, 224, 240, 256, 272, 288, 304, 320, 336, 352, 368, 384, 448, 512,
+         74, 142]   # not multiples of 16: cuFFT with phi_33 from the trace
 
 
 def _close(a, b, name):
