@@ -50,6 +50,8 @@ namespace ppb {
 void Slot::init(int dev) {
   device = dev;
   PPB_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
+  PPB_CUDA(cudaStreamCreateWithFlags(&stream2, cudaStreamNonBlocking));
+  for (cudaEvent_t* e : {&fork_ev, &join_ev}) PPB_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
   for (auto& e : stage_ev) PPB_CUDA(cudaEventCreate(&e));
   for (auto& e : shell_ev) PPB_CUDA(cudaEventCreate(&e));
 }
@@ -169,6 +171,8 @@ Slot::~Slot() {
   release_buffers();
   for (auto& e : stage_ev) if (e) cudaEventDestroy(e);
   for (auto& e : shell_ev) if (e) cudaEventDestroy(e);
+  for (cudaEvent_t e : {fork_ev, join_ev}) if (e) cudaEventDestroy(e);
+  if (stream2) cudaStreamDestroy(stream2);
   if (stream) cudaStreamDestroy(stream);
 }
 
@@ -399,10 +403,6 @@ TuneEntry ppb_ctx::tune_shells(Slot& sl, const ShellArgs& b0, bool comp, bool ad
       float ms = 0.f;
       PPB_CUDA(cudaEventElapsedTime(&ms, ev[0], ev[1]));
       te.gather_ms[slot_of[c]] = std::min(te.gather_ms[slot_of[c]], ms);
-    }
-    for (int o = 0; o < 2; o++) {   // list order, then by descending crossing shell
-      for (int c = 0; c < 4; c++) {
-        PPB_CUDA(cudaEventRecord(ev[0], s));
       if (round == 0 && c == 0) {
         // rows past the pool's end: most peaks are marked overflowed, and the
         // times of what follows would say nothing
@@ -416,6 +416,10 @@ TuneEntry ppb_ctx::tune_shells(Slot& sl, const ShellArgs& b0, bool comp, bool ad
           return te;
         }
       }
+    }
+    for (int o = 0; o < 2; o++) {   // list order, then by descending crossing shell
+      for (int c = 0; c < 4; c++) {
+        PPB_CUDA(cudaEventRecord(ev[0], s));
         collapse_order(sl, b, o == 1);
         launch_shell_collapse(L, b, nsm, sl.walk_per_peak, widths[c]);
         PPB_CUDA(cudaEventRecord(ev[1], s));
@@ -596,12 +600,12 @@ void ppb_ctx::run_shells(Slot& sl, ShellArgs& a, bool comp, bool adaptive, Shell
       if (te.npk > 0) {
         std::lock_guard<std::mutex> lk(sh.cache_mu);
         sh.tune[tkey] = te;
-      }
-    }
-    const int fb = sh.force_brick.load(), fc = sh.force_collapse.load();
         tune_now = false;
       } else {   // the pool was too small: the run below finds its size, then the tuning is repeated
         te = TuneEntry();
+      }
+    }
+    const int fb = sh.force_brick.load(), fc = sh.force_collapse.load();
     const int fo = sh.collapse_order.load();
     const bool corder_on = fo == 1 || (fo == -1 && te.collapse_order);
     if (sh.gather_tex.load() == -1 && !te.gather_tex) b.rec_tex = 0;
@@ -636,11 +640,11 @@ void ppb_ctx::run_shells(Slot& sl, ShellArgs& a, bool comp, bool adaptive, Shell
       const double seen = (double)used / (double)nb;
       PPB_REQUIRE(seen * 1.25 > rpp, "profile pool overflow without growth");
       rpp = seen;
+      set_budget((double)(a.npk - p0));
       continue;
     }
     float k[4];
     for (int e = 0; e < 4; e++) PPB_CUDA(cudaEventElapsedTime(&k[e], sl.shell_ev[e], sl.shell_ev[e + 1]));
-      set_budget((double)(a.npk - p0));
     for (int e = 0; e < 4; e++) s.kms[e] += k[e];
     s.ms += k[0] + k[1] + k[2] + k[3];
     s.pool_rows += used;
@@ -650,14 +654,14 @@ void ppb_ctx::run_shells(Slot& sl, ShellArgs& a, bool comp, bool adaptive, Shell
     std::memcpy(before, c, sizeof(c));
     p0 += nb;
   }
-  s.visits = c[0];
-  for (int i = 0; i < 5; i++) s.dump[i] = c[1 + i];
-  s.guard = c[6];
-  s.akk = c[7];
   // the next call's estimate: the rows per peak of the whole call (the last
   // batch's alone would be the small radii's, and the first batch of the next
   // call would overflow the pool and run twice)
   if (s.batches > 1) rpp = std::max(1.0, (double)s.pool_rows / (double)a.npk);
+  s.visits = c[0];
+  for (int i = 0; i < 5; i++) s.dump[i] = c[1 + i];
+  s.guard = c[6];
+  s.akk = c[7];
   for (int i = 0; i < 16; i++) s.raw[i] = c[i];
   sl.last_shell = s;
   if (st) *st = s;

@@ -105,8 +105,10 @@ __global__ void lpt1_kernel(const float2* __restrict__ dk, float2* __restrict__ 
   }
 }
 
-// phi_ij = -k_i k_j / k^2 delta_k, order 11 22 33 12 13 23, no Nyquist
-// zeroing (LPT.jl:103-128)
+// phi_ij = -k_i k_j / k^2 delta_k, order 11 22 33 12 13 23 (NC = 6) or 11 22
+// 12 13 23 (NC = 5, phi_33 from the trace), no Nyquist zeroing
+// (LPT.jl:103-128)
+template <int NC>
 __global__ void phi_kernel(const float2* __restrict__ dk, float2* __restrict__ out, int n, double mult,
                            double post_scale) {
   const int nh = n / 2 + 1;
@@ -118,10 +120,11 @@ __global__ void phi_kernel(const float2* __restrict__ dk, float2* __restrict__ o
   const float2 d = dk[md.id];
   const int pa[6] = {0, 1, 2, 0, 0, 1}, pb[6] = {0, 1, 2, 1, 2, 2};
 #pragma unroll
-  for (int c = 0; c < 6; c++) {
+  for (int c = 0; c < NC; c++) {
     float2 o = make_float2(0.f, 0.f);
     if (k2 != 0.0) {
-      const double q = (-kv[pa[c]]) * kv[pb[c]] / k2 * post_scale;
+      const int i = NC == 5 && c >= 2 ? c + 1 : c;
+      const double q = (-kv[pa[i]]) * kv[pb[i]] / k2 * post_scale;
       o = make_float2((float)(q * (double)d.x), (float)(q * (double)d.y));
     }
     out[c * M + md.id] = o;
@@ -154,6 +157,17 @@ __global__ void lpt2_kernel(const float2* __restrict__ sk, float2* __restrict__ 
   const double kv[3] = {(double)md.ix * mult, fftfreq(md.iy, n, mult), fftfreq(md.iz, n, mult)};
   const double k2 = kv[0] * kv[0] + kv[1] * kv[1] + kv[2] * kv[2];
   const bool zero = (k2 == 0.0) || md.ix == nh - 1 || md.iy == n / 2 || md.iz == n / 2;
+// the same from phi 11 22 12 13 23 and delta: phi_33 = -(delta + phi_11 +
+// phi_22), since sum_a k_a k_a / k^2 = 1
+__global__ void src2_from_trace_kernel(const float* __restrict__ phi, const float* __restrict__ delta,
+                                       float* __restrict__ out, int64_t N) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < N; i += (int64_t)gridDim.x * blockDim.x) {
+    const float a = phi[i], b = phi[N + i], d = phi[2 * N + i], e = phi[3 * N + i], f = phi[4 * N + i];
+    const float s = a + b, c = -(delta[i] + s);
+    out[i] = a * b + s * c - d * d - e * e - f * f;
+  }
+}
+
   const float2 s = sk[md.id];
 #pragma unroll
   for (int c = 0; c < 3; c++) {
@@ -522,9 +536,10 @@ void launch_lpt1(Launch L, const float2* dk, float2* out, int n, double boxsize,
   PPB_LAUNCHED(*L.count);
 }
 
-void launch_phi(Launch L, const float2* dk, float2* out, int n, double boxsize, double post_scale) {
+void launch_phi(Launch L, const float2* dk, float2* out, int n, double boxsize, double post_scale, int nc) {
   const double dkk = 2.0 * kPi / boxsize;
-  phi_kernel<<<mode_grid(n), 256, 0, L.s>>>(dk, out, n, (n * dkk) / (double)n, post_scale);
+  if (nc == 5) phi_kernel<5><<<mode_grid(n), 256, 0, L.s>>>(dk, out, n, (n * dkk) / (double)n, post_scale);
+  else phi_kernel<6><<<mode_grid(n), 256, 0, L.s>>>(dk, out, n, (n * dkk) / (double)n, post_scale);
   PPB_LAUNCHED(*L.count);
 }
 
@@ -556,6 +571,12 @@ void launch_window_tables(Launch L, float* tab, int n, double boxsize, const dou
 }
 
 void launch_window(Launch L, const float2* dk, float2* out0, float2* out1, int n, const float* tab,
+void launch_src2_from_trace(Launch L, const float* phi, const float* delta, float* out, int64_t N) {
+  const int64_t blocks = std::min<int64_t>((N + 255) / 256, 148 * 32);
+  src2_from_trace_kernel<<<(unsigned)blocks, 256, 0, L.s>>>(phi, delta, out, N);
+  PPB_LAUNCHED(*L.count);
+}
+
                    double post_scale) {
   const int plane = (n / 2 + 1) * n;
   const dim3 grid((unsigned)((plane + 256 * kWinPerThread - 1) / (256 * kWinPerThread)), (unsigned)n, 1);

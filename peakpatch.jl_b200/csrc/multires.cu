@@ -180,7 +180,7 @@ void mr_tile_2lpt_lap(ppb_ctx* ctx, Slot& sl, TileRes& T, int n, double box, flo
     // phi_11, phi_22, phi_33, phi_12, phi_13, phi_23 (:812-821)
     const int pk6[6] = {3, 3, 3, 3, 3, 3}, pa[6] = {1, 2, 3, 1, 1, 2}, pb[6] = {1, 2, 3, 2, 3, 3};
     launch_kspace(L, nullptr, T.dk.as<float2>(), T.kw.as<float2>(), Mk, n, box, pk6, pa, pb, 6, post);
-    PPB_CUFFT(cufftExecC2R(T.c2r6, T.kw.as<cufftComplex>(), T.rw.as<float>()));
+    PPB_CUFFT(cufftExecC2R(T.phi6(sl.stream), T.kw.as<cufftComplex>(), T.rw.as<float>()));
     sl.launches++;
     launch_src2_trace(L, T.delta.as<float>(), T.rw.as<float>(), T.rw.as<float>(), n, n, (int64_t)n * n, N);
     // rfft(src2) into the first phi slot (its transform has consumed it), so
@@ -241,7 +241,7 @@ void mr_coarse_device(ppb_ctx* ctx, Slot& sl, const float* d_noise, int M, doubl
   Launch L{sl.stream, &sl.launches};
   const int64_t N = (int64_t)M * M * M, Mk = (int64_t)(M / 2 + 1) * M * M;
   TileRes& tr = sl.tile_for(M);
-  tr.setup(M, sl.stream);
+  tr.setup(M, sl.stream, sl.stream2);
   PPB_CUDA(cudaMemcpyAsync(tr.delta.p, d_noise, N * 4, cudaMemcpyDeviceToDevice, sl.stream));
   PPB_CUFFT(cufftExecR2C(tr.r2c, tr.delta.as<float>(), tr.dk.as<cufftComplex>()));
   sl.launches++;
@@ -263,7 +263,7 @@ void mr_coarse_device(ppb_ctx* ctx, Slot& sl, const float* d_noise, int M, doubl
   if (ilpt >= 2) {  // the 2LPT source and displacements (:635-659)
     const int pk6[6] = {3, 3, 3, 3, 3, 3}, pa[6] = {1, 2, 3, 1, 1, 2}, pb[6] = {1, 2, 3, 2, 3, 3};
     launch_kspace(L, amp, tr.dk.as<float2>(), tr.kw.as<float2>(), Mk, M, boxsize_full, pk6, pa, pb, 6, post);
-    PPB_CUFFT(cufftExecC2R(tr.c2r6, tr.kw.as<cufftComplex>(), tr.rw.as<float>()));
+    PPB_CUFFT(cufftExecC2R(tr.phi6(sl.stream), tr.kw.as<cufftComplex>(), tr.rw.as<float>()));
     sl.launches++;
     launch_src2_trace(L, o, tr.rw.as<float>(), tr.rw.as<float>(), M, M, (int64_t)M * M, N);
     PPB_CUFFT(cufftExecR2C(tr.r2c, tr.rw.as<float>(), tr.dk.as<cufftComplex>()));
@@ -336,7 +336,7 @@ void finish_out(float* dst, const float* dev, size_t bytes, cudaStream_t s) {
 TileRes& periodic_setup(ppb_ctx* ctx, const float* delta_tile, int n) {
   Slot& sl = ctx->sync;
   TileRes& tr = sl.tile_for(n);
-  tr.setup(n, sl.stream);
+  tr.setup(n, sl.stream, sl.stream2);
   const int64_t N = (int64_t)n * n * n;
   PPB_CUDA(cudaMemcpyAsync(tr.delta.p, delta_tile, N * 4, cudaMemcpyDefault, sl.stream));
   return tr;

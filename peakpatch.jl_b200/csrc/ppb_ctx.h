@@ -17,7 +17,12 @@ namespace ppb {
 // plans and device buffers for one grid size n
 struct TileRes {
   int n = 0;
-  cufftHandle r2c = 0, c2r1 = 0, c2r2 = 0, c2r3 = 0, c2r6 = 0;
+  // (c2r2, c2r5: sizes without the fused transforms; c2r6: made by phi6)
+  cufftHandle r2c = 0, c2r1 = 0, c2r2 = 0, c2r3 = 0, c2r5 = 0, c2r6 = 0;
+  // small grids: plans on the slot's second stream, with their own buffers
+  // (0 where one stream is used)
+  cufftHandle c2r1b = 0, c2r2b = 0, c2r3b = 0;
+  DevBuf kwb, rwb;
   // in-place inverse C2C of contiguous n x n (kz, ky) planes, batched over
   // the n/2+1 kx: the filter bank's transforms before the fused x pass (0
   // where unsupported)
@@ -32,7 +37,9 @@ struct TileRes {
   // bank): they live exactly as long as the plans whose kernels they launch
   std::map<std::pair<int, int64_t>, cudaGraphExec_t> graphs;
   ~TileRes();
-  void setup(int n, cudaStream_t s);
+  void setup(int n, cudaStream_t s, cudaStream_t s2);
+  // the six-field plan of the multi-resolution stages (outside capture)
+  cufftHandle phi6(cudaStream_t s);
   // the fused filter bank's plans, twiddle buffer and kernel attribute, made
   // the first time a filter bank of this size takes that path (outside capture)
   void setup_fused(cudaStream_t s);
@@ -91,6 +98,10 @@ constexpr size_t kStubKeep = (size_t)4 << 30;   // stub buffers kept between cal
 struct Slot {
   int device = 0;
   cudaStream_t stream = nullptr;
+  // small grids: work beside the stream's, always joined back into it (fork
+  // and join events) before the phase ends
+  cudaStream_t stream2 = nullptr;
+  cudaEvent_t fork_ev = nullptr, join_ev = nullptr;
   int64_t launches = 0;
   cudaEvent_t stage_ev[5] = {};
   cudaEvent_t shell_ev[5] = {};

@@ -271,8 +271,11 @@ void launch_noise(Launch L, float* out, int64_t n, uint64_t seed);
 void launch_convolve(Launch L, float2* nk, int n, double boxsize, const double* lk, const double* lp,
                      int np, double pk_scale, double post_scale);
 void launch_lpt1(Launch L, const float2* dk, float2* out, int n, double boxsize, double post_scale);
-void launch_phi(Launch L, const float2* dk, float2* out, int n, double boxsize, double post_scale);
+// nc = 6: phi 11 22 33 12 13 23; nc = 5: without phi_33, which
+// launch_src2_from_trace takes from delta
+void launch_phi(Launch L, const float2* dk, float2* out, int n, double boxsize, double post_scale, int nc);
 void launch_src2(Launch L, const float* phi, float* out, int64_t N);
+void launch_src2_from_trace(Launch L, const float* phi, const float* delta, float* out, int64_t N);
 void launch_lpt2(Launch L, const float2* s2k, float2* out, int n, double boxsize, double post_scale);
 void launch_lapd(Launch L, const float2* dk, float2* out, int n, double boxsize, float post_scale);
 // window tables: per filter f, window_table_size(n) floats W_wsmooth, then as

@@ -264,22 +264,41 @@ TileRes::~TileRes() {
   for (auto& g : graphs)   // before the plans whose kernels they launch
     if (g.second) cudaGraphExecDestroy(g.second);
   graphs.clear();
-  for (cufftHandle h : {r2c, c2r1, c2r2, c2r3, c2r6, yz1})
+  for (cufftHandle h : {r2c, c2r1, c2r2, c2r3, c2r5, c2r6, yz1, c2r1b, c2r2b, c2r3b})
     if (h) cufftDestroy(h);
 }
 
-void TileRes::setup(int nn, cudaStream_t s) {
+// largest grid whose transforms take a second stream: up to here a kernel of
+// one field leaves part of the device idle (run_tile 142^3 4.00 -> 3.64 ms,
+// fields 142^3 1.69 -> 1.56 with phi_33 from the trace, 128^3 tile 1.94 ->
+// 1.87); the kernels of a 192^3 field fill it
+constexpr int kTwoStreams = 160;
+
+void TileRes::setup(int nn, cudaStream_t s, cudaStream_t s2) {
   if (n == nn) return;
-  for (cufftHandle* h : {&r2c, &c2r1, &c2r2, &c2r3, &c2r6, &yz1})
+  for (cufftHandle* h : {&r2c, &c2r1, &c2r2, &c2r3, &c2r5, &c2r6, &yz1, &c2r1b, &c2r2b, &c2r3b})
     if (*h) { cufftDestroy(*h); *h = 0; }
   n = nn;
   const int64_t N = (int64_t)n * n * n, M = (int64_t)(n / 2 + 1) * n * n;
   r2c = make_plan(n, CUFFT_R2C, 1);
   c2r1 = make_plan(n, CUFFT_C2R, 1);
-  c2r2 = make_plan(n, CUFFT_C2R, 2);
   c2r3 = make_plan(n, CUFFT_C2R, 3);
-  c2r6 = make_plan(n, CUFFT_C2R, 6);
-  for (cufftHandle h : {r2c, c2r1, c2r2, c2r3, c2r6}) PPB_CUFFT(cufftSetStream(h, s));
+  if (!fft_supported(n)) {   // the twin's and 2LPT's full transforms
+    c2r2 = make_plan(n, CUFFT_C2R, 2);
+    c2r5 = make_plan(n, CUFFT_C2R, 5);
+  }
+  for (cufftHandle h : {r2c, c2r1, c2r2, c2r3, c2r5})
+    if (h) PPB_CUFFT(cufftSetStream(h, s));
+
+  if (n <= kTwoStreams) {
+    c2r1b = make_plan(n, CUFFT_C2R, 1);
+    c2r3b = make_plan(n, CUFFT_C2R, 3);
+    if (!fft_supported(n)) c2r2b = make_plan(n, CUFFT_C2R, 2);
+    for (cufftHandle h : {c2r1b, c2r2b, c2r3b})
+      if (h) PPB_CUFFT(cufftSetStream(h, s2));
+    kwb.ensure(3 * M * 8);
+    rwb.ensure(2 * N * 4);
+  }
 
   delta.ensure(N * 4);
   dk.ensure(M * 8);
@@ -298,9 +317,17 @@ void TileRes::setup(int nn, cudaStream_t s) {
   }
 }
 
+cufftHandle TileRes::phi6(cudaStream_t s) {
+  if (!c2r6) {
+    c2r6 = make_plan(n, CUFFT_C2R, 6);
+    PPB_CUFFT(cufftSetStream(c2r6, s));
+  }
+  return c2r6;
+}
+
 size_t TileRes::bytes() const {
   size_t b = 0;
-  for (const DevBuf* d : {&delta, &dk, &psi, &psi2, &lapd, &aos, &kw, &rw, &mask, &count, &wtab, &keys, &vals, &ff,
+  for (const DevBuf* d : {&delta, &dk, &psi, &psi2, &lapd, &aos, &kw, &rw, &kwb, &rwb, &mask, &count, &wtab, &keys, &vals, &ff,
                           &lap, &keys_s, &vals_s, &tmp, &p_lin, &p_Rf, &p_ir2, &p_np, &p_Z, &p_fc, &p_FcRf, &p_d2Rf,
                           &p_pos, &res, &flags, &offs, &rec, &rthl, &xtw})
     b += d->bytes;
@@ -482,6 +509,17 @@ void setup_run(Run& r, ppb_ctx* ctx, Slot& sl, const ppb_tile_params* p, const d
   PPB_CUDA(cudaMemcpyAsync(sl.filt_ir2.p, fir2.data(), nfilt * 4, cudaMemcpyHostToDevice, r.s));
 }
 
+// the slot's second stream starts from here on / the slot's stream waits for
+// it; both legal while the slot's stream is being captured
+void fork(Slot& sl) {
+  PPB_CUDA(cudaEventRecord(sl.fork_ev, sl.stream));
+  PPB_CUDA(cudaStreamWaitEvent(sl.stream2, sl.fork_ev, 0));
+}
+void join(Slot& sl) {
+  PPB_CUDA(cudaEventRecord(sl.join_ev, sl.stream2));
+  PPB_CUDA(cudaStreamWaitEvent(sl.stream, sl.join_ev, 0));
+}
+
 // phase 1 (Pipeline.jl:90-140, MultiTile.jl:157-194): Threefry noise -> R2C
 // -> sqrt(P) -> C2R = delta; delta_k = R2C(delta), projected Hermitian;
 // 1LPT, 2LPT and the Laplacian field, all on the n^3 grid of `box`
@@ -504,14 +542,25 @@ void fields_phase(Run& r, TileRes& T, int n, double box) {
   // one Hermitian projection of delta_k: every filter output W(|k|) delta_k
   // (and k^2 W delta_k) is then Hermitian as it stands
   launch_hermitise(L, dkp, n, 1);
-  // 1LPT
-  launch_lpt1(L, dkp, kw, n, box, inv_n3);
-  launch_hermitise(L, kw, n, 3);
-  if (r.plain) {
-    for (int c = 0; c < 3; c++)
-      PPB_CUFFT(cufftExecC2R(T.c2r1, (cufftComplex*)(kw + c * M), T.psi.as<cufftReal>() + c * N));
+  // 1LPT; on small grids beside 2LPT and the Laplacian, on the slot's second
+  // stream
+  const bool two = T.c2r3b && !r.plain;
+  if (two) {
+    fork(*r.sl);
+    const Launch L2{r.sl->stream2, L.count};
+    float2* kb = T.kwb.as<float2>();
+    launch_lpt1(L2, dkp, kb, n, box, inv_n3);
+    launch_hermitise(L2, kb, n, 3);
+    PPB_CUFFT(cufftExecC2R(T.c2r3b, (cufftComplex*)kb, T.psi.as<cufftReal>()));
   } else {
-    PPB_CUFFT(cufftExecC2R(T.c2r3, (cufftComplex*)kw, T.psi.as<cufftReal>()));
+    launch_lpt1(L, dkp, kw, n, box, inv_n3);
+    launch_hermitise(L, kw, n, 3);
+    if (r.plain) {
+      for (int c = 0; c < 3; c++)
+        PPB_CUFFT(cufftExecC2R(T.c2r1, (cufftComplex*)(kw + c * M), T.psi.as<cufftReal>() + c * N));
+    } else {
+      PPB_CUFFT(cufftExecC2R(T.c2r3, (cufftComplex*)kw, T.psi.as<cufftReal>()));
+    }
   }
   // psi2 and the Laplacian feed no collapse decision: for the sizes of
   // k_fft.cu they take the fused transforms (fields with 2LPT and Laplacian,
@@ -525,14 +574,18 @@ void fields_phase(Run& r, TileRes& T, int n, double box) {
     fft_work_arrays(T, n, w);
     launch_lpt2_fused(L, dkp, T.delta.as<float>(), w, T.xtw.as<float2>(), T.psi2.as<float>(), n, box, true);
   } else if (p->ilpt >= 2) {
-    launch_phi(L, dkp, kw, n, box, inv_n3);
-    launch_hermitise(L, kw, n, 6);
+    // src2 into the lapd buffer; the plain path transforms all six phi one by
+    // one, the batched one five
+    const int nc = r.plain ? 6 : 5;
+    launch_phi(L, dkp, kw, n, box, inv_n3, nc);
+    launch_hermitise(L, kw, n, nc);
     if (r.plain) {
       for (int c = 0; c < 6; c++) PPB_CUFFT(cufftExecC2R(T.c2r1, (cufftComplex*)(kw + c * M), rw + c * N));
+      launch_src2(L, rw, T.lapd.as<float>(), N);
     } else {
-      PPB_CUFFT(cufftExecC2R(T.c2r6, (cufftComplex*)kw, rw));
+      PPB_CUFFT(cufftExecC2R(T.c2r5, (cufftComplex*)kw, rw));
+      launch_src2_from_trace(L, rw, T.delta.as<float>(), T.lapd.as<float>(), N);
     }
-    launch_src2(L, rw, T.lapd.as<float>(), N);   // lapd buffer as scratch for src2
     PPB_CUFFT(cufftExecR2C(T.r2c, T.lapd.as<cufftReal>(), (cufftComplex*)kw));
     launch_lpt2(L, kw, kw + M, n, box, inv_n3);
     launch_hermitise(L, kw + M, n, 3);
@@ -553,6 +606,7 @@ void fields_phase(Run& r, TileRes& T, int n, double box) {
     launch_hermitise(L, kw, n, 1);
     PPB_CUFFT(cufftExecC2R(T.c2r1, (cufftComplex*)kw, T.lapd.as<cufftReal>()));
   }
+  if (two) join(*r.sl);
 }
 
 // phase 2 (Pipeline.jl:144-196, MultiTile.jl:218-275): per filter, largest
@@ -629,17 +683,29 @@ int64_t peaks_phase(Run& r, TileRes& T, int n, double box, const std::vector<Win
                        r.ffc.empty() ? wins[0].fcrit : r.ffc[f], (unsigned long long)f, pb);
         } else {
           const bool lap = r.want_lap && !twin;   // the full twin field, read by the search
-          launch_window(L, dkp, kw, lap ? kw + M : nullptr, n, tab, inv_n3);
-          if (lap && !r.plain) {
-            PPB_CUFFT(cufftExecC2R(T.c2r2, (cufftComplex*)kw, rw));
-          } else {
-            PPB_CUFFT(cufftExecC2R(T.c2r1, (cufftComplex*)kw, rw));
-            if (lap) PPB_CUFFT(cufftExecC2R(T.c2r1, (cufftComplex*)(kw + M), rw + N));
+          // smoothed field (and twin) of filter f; on small grids the odd
+          // filters' on the second stream, beside the even ones'
+          auto smooth = [&](const Launch& Lf, int g, float2* k, float* x, cufftHandle one, cufftHandle pair) {
+            launch_window(Lf, dkp, k, lap ? k + M : nullptr, n, T.wtab.as<float>() + (size_t)g * 2 * qn, inv_n3);
+            if (lap && !r.plain) {
+              PPB_CUFFT(cufftExecC2R(pair, (cufftComplex*)k, x));
+            } else {
+              PPB_CUFFT(cufftExecC2R(one, (cufftComplex*)k, x));
+              if (lap) PPB_CUFFT(cufftExecC2R(one, (cufftComplex*)(k + M), x + N));
+            }
+          };
+          const bool two = T.c2r1b && !r.plain, second = two && f % 2 == 1;
+          if (two && f % 2 == 0 && f + 1 < r.nfilt) {
+            fork(*r.sl);
+            smooth(Launch{r.sl->stream2, L.count}, f + 1, T.kwb.as<float2>(), T.rwb.as<float>(), T.c2r1b, T.c2r2b);
           }
+          if (second) join(*r.sl);
+          else smooth(L, f, kw, rw, T.c2r1, T.c2r2);
+          const float* x = second ? T.rwb.as<float>() : rw;
           for (size_t t = 0; t < wins.size(); t++) {
             const Win& w = wins[t];
-            launch_peakfind(L, rw + w.off, lap ? rw + N + w.off : nullptr, T.mask.as<uint8_t>() + w.off, nm, nm, nm,
-                            n, (int64_t)n * n, p->nbuff, r.ffc.empty() ? w.fcrit : r.ffc[f],
+            launch_peakfind(L, x + w.off, lap ? x + N + w.off : nullptr, T.mask.as<uint8_t>() + w.off, nm, nm, nm, n,
+                            (int64_t)n * n, p->nbuff, r.ffc.empty() ? w.fcrit : r.ffc[f],
                             ((unsigned long long)t << r.fbits) | (unsigned long long)f, pb);
           }
         }
@@ -838,7 +904,7 @@ void peak_find_tile_core(ppb_ctx* ctx, Slot& sl, const float* delta, int n, cons
   PPB_CUDA(cudaMemcpyAsync(sl.filt_Rf.p, r.Rf.data(), nfilt * 8, cudaMemcpyHostToDevice, r.s));
   PPB_CUDA(cudaMemsetAsync(sl.filt_ir2.p, 0, nfilt * 4, r.s));
   TileRes& T = sl.tile_for(n);
-  T.setup(n, r.s);
+  T.setup(n, r.s, r.sl->stream2);
   if (T.cap == 0) T.ensure_peaks(initial_peak_capacity(N));
   // rfft(delta) once, projected Hermitian as run_tile's delta_k
   PPB_CUDA(cudaMemcpyAsync(T.delta.p, delta, N * 4, cudaMemcpyDefault, r.s));
@@ -902,7 +968,7 @@ void generate_fields_core(ppb_ctx* ctx, Slot& sl, const ppb_tile_params* p, floa
   r.plain = p->plain != 0;
   r.want_lap = p->ioutshear >= 1;
   TileRes& T = sl.tile_for(n);
-  T.setup(n, r.s);
+  T.setup(n, r.s, r.sl->stream2);
   fields_phase(r, T, n, p->boxsize);
   if (delta) copy_out(delta, T.delta.p, N * 4, r.s);
   if (psi) copy_out(psi, T.psi.p, 3 * N * 4, r.s);
@@ -921,7 +987,7 @@ void run_tile_core(ppb_ctx* ctx, Slot& sl, const ppb_tile_params* p, const doubl
   Run r;
   setup_run(r, ctx, sl, p, Rf_in, nfilt, box / n);
   TileRes& T = sl.tile_for(n);
-  T.setup(n, r.s);
+  T.setup(n, r.s, r.sl->stream2);
   T.aos.ensure(pack_bytes(n));
   if (T.cap == 0) T.ensure_peaks(initial_peak_capacity(N));
   cudaEvent_t* ev = sl.stage_ev;
@@ -1032,7 +1098,7 @@ void run_multitile_core(ppb_ctx* ctx, Slot& sl, const ppb_tile_params* p, const 
     wins[t].fcrit = (float)fc;
   }
   TileRes& T = sl.tile_for(n);
-  T.setup(n, r.s);
+  T.setup(n, r.s, r.sl->stream2);
   if (T.cap == 0) T.ensure_peaks(initial_peak_capacity(N));
   sl.tcen.ensure(tcen.size() * 8);
   PPB_CUDA(cudaMemcpyAsync(sl.tcen.p, tcen.data(), tcen.size() * 8, cudaMemcpyHostToDevice, r.s));
@@ -1221,7 +1287,7 @@ void run_multitile_split_core(ppb_ctx* ctx, Slot& sl, const ppb_tile_params* p, 
   mr_coarse_device(ctx, sl, cnoise, M, box_full, 1, 0, cf, fs);
   launch_interleave4(r.L, cf4, cf, fs, Mc);
   TileRes& T = sl.tile_for(nm);
-  T.setup(nm, r.s);
+  T.setup(nm, r.s, r.sl->stream2);
   T.aos.ensure(pack_bytes(nm));
   if (T.cap == 0) T.ensure_peaks(initial_peak_capacity(Nt));
   const int nf = p->ioutshear >= 1 ? 33 : 11;
