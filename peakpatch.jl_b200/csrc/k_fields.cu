@@ -147,16 +147,6 @@ __global__ void src2_kernel(const float* __restrict__ phi, float* __restrict__ o
   }
 }
 
-// psi2_c = -i k_c / k^2 src2_k with Nyquist zeroing (LPT.jl:155-182)
-__global__ void lpt2_kernel(const float2* __restrict__ sk, float2* __restrict__ out, int n, double mult,
-                            double post_scale) {
-  const int nh = n / 2 + 1;
-  const Mode md = mode_of(n, nh);
-  if (!md.ok) return;
-  const int64_t M = (int64_t)nh * n * n;
-  const double kv[3] = {(double)md.ix * mult, fftfreq(md.iy, n, mult), fftfreq(md.iz, n, mult)};
-  const double k2 = kv[0] * kv[0] + kv[1] * kv[1] + kv[2] * kv[2];
-  const bool zero = (k2 == 0.0) || md.ix == nh - 1 || md.iy == n / 2 || md.iz == n / 2;
 // the same from phi 11 22 12 13 23 and delta: phi_33 = -(delta + phi_11 +
 // phi_22), since sum_a k_a k_a / k^2 = 1
 __global__ void src2_from_trace_kernel(const float* __restrict__ phi, const float* __restrict__ delta,
@@ -168,6 +158,16 @@ __global__ void src2_from_trace_kernel(const float* __restrict__ phi, const floa
   }
 }
 
+// psi2_c = -i k_c / k^2 src2_k with Nyquist zeroing (LPT.jl:155-182)
+__global__ void lpt2_kernel(const float2* __restrict__ sk, float2* __restrict__ out, int n, double mult,
+                            double post_scale) {
+  const int nh = n / 2 + 1;
+  const Mode md = mode_of(n, nh);
+  if (!md.ok) return;
+  const int64_t M = (int64_t)nh * n * n;
+  const double kv[3] = {(double)md.ix * mult, fftfreq(md.iy, n, mult), fftfreq(md.iz, n, mult)};
+  const double k2 = kv[0] * kv[0] + kv[1] * kv[1] + kv[2] * kv[2];
+  const bool zero = (k2 == 0.0) || md.ix == nh - 1 || md.iy == n / 2 || md.iz == n / 2;
   const float2 s = sk[md.id];
 #pragma unroll
   for (int c = 0; c < 3; c++) {
@@ -549,6 +549,12 @@ void launch_src2(Launch L, const float* phi, float* out, int64_t N) {
   PPB_LAUNCHED(*L.count);
 }
 
+void launch_src2_from_trace(Launch L, const float* phi, const float* delta, float* out, int64_t N) {
+  const int64_t blocks = std::min<int64_t>((N + 255) / 256, 148 * 32);
+  src2_from_trace_kernel<<<(unsigned)blocks, 256, 0, L.s>>>(phi, delta, out, N);
+  PPB_LAUNCHED(*L.count);
+}
+
 void launch_lpt2(Launch L, const float2* s2k, float2* out, int n, double boxsize, double post_scale) {
   const double dkk = 2.0 * kPi / boxsize;
   lpt2_kernel<<<mode_grid(n), 256, 0, L.s>>>(s2k, out, n, (n * dkk) / (double)n, post_scale);
@@ -571,12 +577,6 @@ void launch_window_tables(Launch L, float* tab, int n, double boxsize, const dou
 }
 
 void launch_window(Launch L, const float2* dk, float2* out0, float2* out1, int n, const float* tab,
-void launch_src2_from_trace(Launch L, const float* phi, const float* delta, float* out, int64_t N) {
-  const int64_t blocks = std::min<int64_t>((N + 255) / 256, 148 * 32);
-  src2_from_trace_kernel<<<(unsigned)blocks, 256, 0, L.s>>>(phi, delta, out, N);
-  PPB_LAUNCHED(*L.count);
-}
-
                    double post_scale) {
   const int plane = (n / 2 + 1) * n;
   const dim3 grid((unsigned)((plane + 256 * kWinPerThread - 1) / (256 * kWinPerThread)), (unsigned)n, 1);
