@@ -340,7 +340,10 @@ __global__ void pack_kernel(float4* __restrict__ aos, FieldWindow w, int n) {
     if (a < n && c < n) tile[r][threadIdx.x] = w.delta[src(c, a, b)];
   }
   __syncthreads();
-  for (int r = threadIdx.y; r < 32; r += blockDim.y) {
+  // four rows' loads in flight per thread (384^3 0.85 -> 0.62 ms)
+#pragma unroll
+  for (int r0 = 0; r0 < 32; r0 += 8) {   // blockDim.y = 8
+    const int r = r0 + threadIdx.y;
     const int a = a0 + threadIdx.x, c = c0 + r;
     if (a >= n || c >= n) continue;
     const int64_t g = src(a, b, c);
