@@ -1537,7 +1537,7 @@ __device__ __forceinline__ void coop_sums(const ShellArgs& a, bool act, long lon
 // stays in the loop until the warp's last walk ends.  With 32 lanes the first
 // round takes kFirst steps, since most walks of a single-redshift tile end
 // there.
-// Measured against four lanes that each read their own window: 13,600 peaks
+// Measured against four lanes that each read their own window: 23,070 peaks
 // of a 128^3 tile 0.44 -> 0.28 ms, four lightcone tiles of 192^3 5.3 -> 3.9;
 // one and two lanes per peak keep their own windows, being faster so on full
 // batches (384^3, two lanes 3.15 ms; with the shared sums 3.55) and on the
@@ -2016,8 +2016,9 @@ int shell_collapseq_blocks(int nsm) {
 }
 
 int shell_collapse_width(int64_t npk, int nsm, double walk_steps_per_peak) {
-  // a warp per peak for small batches (7,002 peaks: 0.41 ms with four threads
-  // each reading its own window, 0.28 so), 4 threads per peak while 4 per peak still fit about 24 warps per SM or
+  // a warp per peak for small batches (against four threads per peak: 2,944
+  // peaks 0.111 -> 0.057 ms, 5,820 peaks 0.154 -> 0.117, 9,816 peaks 0.145 ->
+  // 0.162), 4 threads per peak while 4 per peak still fit about 24 warps per SM or
   // when walks are long (more than 8 steps per peak in the previous batch:
   // the lightcone), else 2 or 1 (the device is full and the latency hidden)
   const int64_t full = (int64_t)nsm * 24 * 32;
@@ -2038,7 +2039,7 @@ void launch_shell_collapse(Launch L, const ShellArgs& a, int nsm, double walk_st
   if (w != 1 && w != 2 && w != 4) w = shell_collapse_width(a.npk, nsm, walk_steps_per_peak);
   const int lg = w == 32 ? 5 : w == 4 ? 2 : w - 1;
   const int64_t blocks = ((a.npk << lg) + 127) / 128;
-constexpr int64_t kWarpPeaks = 12000;   // 81 warps per SM
+constexpr int64_t kWarpPeaks = 8000;   // 54 warps per SM
   if (blocks == 0) return;
   if (w == 32) collapse_lanes_kernel<32><<<(unsigned)blocks, 128, 0, L.s>>>(a);
   else if (w == 4) collapse_lanes_kernel<4><<<(unsigned)blocks, 128, 0, L.s>>>(a);
