@@ -423,6 +423,7 @@ class Context:
         nz, ny, nx = d.shape
         self._check(self.L.ppb_set_collapse_table(self.h, _p(d), nx, ny, nz, t.X1, t.X2, t.Y1, t.Y2, t.Z1, t.Z2))
         self._table_key = key
+        self._table_ref = t.data   # the key names it by its id: no other array may take that
 
     def set_pk_table(self, k: np.ndarray, pk: np.ndarray):
         k = np.ascontiguousarray(k, np.float64)
