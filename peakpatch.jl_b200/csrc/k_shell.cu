@@ -1528,9 +1528,10 @@ __device__ __forceinline__ void coop_sums(const ShellArgs& a, bool act, long lon
 }
 
 // QT threads per peak (QT = 4 or 32; 32 / QT peaks per warp): the inward walk
-// (RadialShell.jl:566-699) evaluates up to QT consecutive steps per round, lane q of a peak taking step base + q (mp = m0 - step; step 0 is the
-// m0 step, whose zvir is forced to -1), and the peak takes the first step
-// that collapses; the step before it comes from the lane to its left or, for
+// (RadialShell.jl:566-699) evaluates up to QT consecutive steps per round,
+// lane q of a peak taking step base + q (mp = m0 - step; step 0 is the m0
+// step, whose zvir is forced to -1), and the peak takes the first step that
+// collapses; the step before it comes from the lane to its left or, for
 // q = 0, from the previous round's last step.  Only the strain is needed to
 // walk; the gradients are formed for the two steps a collapse interpolates
 // between.  The row sums run on the whole warp (coop_strain), so every lane
@@ -2015,13 +2016,15 @@ int shell_collapseq_blocks(int nsm) {
   return nsm * per_sm;
 }
 
+constexpr int64_t kWarpPeaks = 8000;   // 54 warps per SM
 int shell_collapse_width(int64_t npk, int nsm, double walk_steps_per_peak) {
   // a warp per peak for small batches (against four threads per peak: 2,944
   // peaks 0.111 -> 0.057 ms, 5,820 peaks 0.154 -> 0.117, 9,816 peaks 0.145 ->
-  // 0.162), 4 threads per peak while 4 per peak still fit about 24 warps per SM or
-  // when walks are long (more than 8 steps per peak in the previous batch:
+  // 0.162), 4 threads per peak while 4 per peak still fit about 24 warps per
+  // SM or when walks are long (more than 8 steps per peak in the previous batch:
   // the lightcone), else 2 or 1 (the device is full and the latency hidden)
   const int64_t full = (int64_t)nsm * 24 * 32;
+  if (npk <= kWarpPeaks) return 32;
   if (walk_steps_per_peak > 8.0 || npk * 4 <= full) return 4;
   return npk * 2 <= full ? 2 : 1;
 }
@@ -2039,14 +2042,12 @@ void launch_shell_collapse(Launch L, const ShellArgs& a, int nsm, double walk_st
   if (w != 1 && w != 2 && w != 4) w = shell_collapse_width(a.npk, nsm, walk_steps_per_peak);
   const int lg = w == 32 ? 5 : w == 4 ? 2 : w - 1;
   const int64_t blocks = ((a.npk << lg) + 127) / 128;
-constexpr int64_t kWarpPeaks = 8000;   // 54 warps per SM
   if (blocks == 0) return;
   if (w == 32) collapse_lanes_kernel<32><<<(unsigned)blocks, 128, 0, L.s>>>(a);
   else if (w == 4) collapse_lanes_kernel<4><<<(unsigned)blocks, 128, 0, L.s>>>(a);
   else if (w == 2) collapse_kernel<2><<<(unsigned)blocks, 128, 0, L.s>>>(a);
   else collapse1_kernel<<<(unsigned)blocks, 128, 0, L.s>>>(a);
   PPB_LAUNCHED(*L.count);
-  if (npk <= kWarpPeaks) return 32;
 }
 
 void launch_shell_zhalf(Launch L, const ShellArgs& a) {
