@@ -611,6 +611,54 @@ __device__ __forceinline__ int sum_chunk(const ShellArgs& a, int ck, int cnt, in
   return nsh;
 }
 
+// a shell's row from its chunks' partials (columns k0 .. k0 + nk - 1)
+__device__ __forceinline__ void write_row(double* dst, const double* part, int k0, int nk, double r, double fb,
+                                          double nsh) {
+  double t[NACC];
+#pragma unroll
+  for (int v = 1; v < NACC; v++) t[v] = 0.0;
+  for (int k = k0; k < k0 + nk; k++) {
+#pragma unroll
+    for (int v = 1; v < NACC; v++) t[v] += part[v * 32 + k];
+  }
+  const double ir = 1.0 / r;   // one division; the products differ from t / r by at most an ulp
+  double row[ROW];
+#pragma unroll
+  for (int v = 0; v < ROW; v++) row[v] = 0.0;
+  row[R_FBAR] = fb;
+  row[R_N] = nsh;
+#pragma unroll
+  for (int L = 0; L < 3; L++) {
+    row[R_S + L] = t[1 + L];
+    row[R_S2 + L] = t[4 + L];
+    row[R_G + L] = t[7 + L] * ir;
+    row[R_GF + L] = t[10 + L] * ir;
+  }
+  row[R_Q + 0] = (2.0 * t[13]) * ir;
+  row[R_Q + 1] = (2.0 * t[14]) * ir;
+  row[R_Q + 2] = (2.0 * t[15]) * ir;
+  row[R_Q + 3] = t[16] * ir;
+  row[R_Q + 4] = t[17] * ir;
+  row[R_Q + 5] = t[18] * ir;
+  double2* d2 = reinterpret_cast<double2*>(dst);
+#pragma unroll
+  for (int v = 0; v < ROW / 2; v++) d2[v] = make_double2(row[2 * v], row[2 * v + 1]);
+}
+
+// value v of the peak cell's row (shell 1): c0 = (delta, deltaT, psi_z,
+// psi2_x), c1 = (psi_x, psi_y, psi2_y, psi2_z)
+__device__ __forceinline__ double centre_row(int v, const float4& c0, const float4& c1) {
+  if (v == R_FBAR) return (double)c0.x;
+  if (v == R_N) return 1.0;
+  if (v == R_S) return (double)c1.x;
+  if (v == R_S + 1) return (double)c1.y;
+  if (v == R_S + 2) return (double)c0.z;
+  if (v == R_S2) return (double)c0.w;
+  if (v == R_S2 + 1) return (double)c1.z;
+  if (v == R_S2 + 2) return (double)c1.w;
+  return 0.0;
+}
+
 template <bool COMP, bool ADAPTIVE, int SRC>
 __device__ void gather_one(const ShellArgs& a, int64_t p, double* stage, double* part, Ring* ring) {
   const int lane = threadIdx.x & 31;
@@ -638,25 +686,14 @@ __device__ void gather_one(const ShellArgs& a, int64_t p, double* stage, double*
   // cells past the first cell of shell mmax + 1 are not summed (a peak with a
   // shorter list reads only its own shells; the list's last shell is never
   // finalised, RadialShell.jl:386-390)
-  const int cell_lim = __ldg(a.sh_start + mmax);
+  int cell_lim = __ldg(a.sh_start + mmax);
   const int m0_init = gq.x, mrf = gq.y, mupp_rf = gq.w;
 
   // ---- the peak cell (shell 1) ------------------------------------------
   const float4* __restrict__ aos = a.aos;
   float4 c0, c1;
   ldg_record(aos + 2 * lin, c0, c1);
-  if (lane < ROW) {   // c0 = (delta, deltaT, psi_z, psi2_x), c1 = (psi_x, psi_y, psi2_y, psi2_z)
-    double v = 0.0;
-    if (lane == R_FBAR) v = (double)c0.x;
-    else if (lane == R_N) v = 1.0;
-    else if (lane == R_S) v = (double)c1.x;
-    else if (lane == R_S + 1) v = (double)c1.y;
-    else if (lane == R_S + 2) v = (double)c0.z;
-    else if (lane == R_S2) v = (double)c0.w;
-    else if (lane == R_S2 + 1) v = (double)c1.z;
-    else if (lane == R_S2 + 2) v = (double)c1.w;
-    stage[ROW + lane] = v;
-  }
+  if (lane < ROW) stage[ROW + lane] = centre_row(lane, c0, c1);
   const bool inside = (pc.w & 2) != 0;
   int state = 0;          // 0 unknown, 1 inward, 2 crossing found
   int mcross = 0;
@@ -668,55 +705,30 @@ __device__ void gather_one(const ShellArgs& a, int64_t p, double* stage, double*
   for (int g = 0; g < a.ngroups; g++) {
     const int base = __ldg(a.grp_a + g);
     if (base > mmax || (mtarget >= 0 && base > mtarget)) break;
-    const int gend = min(__ldg(a.grp_b + g), mmax);
+    int gend = min(__ldg(a.grp_b + g), mmax);
+    if (mtarget >= 0) gend = min(gend, mtarget);
     const int c0g = __ldg(a.grp_c + g), ncg = __ldg(a.grp_c + g + 1) - c0g;
     // (a) lane l sums chunk c0g + l into the shared partial table
-    if (lane < ncg) {
-      const int s0 = __ldg(a.ck_s + c0g + lane), cnt = s0 < cell_lim ? __ldg(a.ck_n + c0g + lane) : 0;
-      visits += sum_chunk<COMP, SRC>(a, c0g + lane, cnt, lin, inside, pi, pj, pk, part, lane, ring);
-    }
+    if (lane < ncg && __ldg(a.ck_s + c0g + lane) < cell_lim)
+      visits += sum_chunk<COMP, SRC>(a, c0g + lane, __ldg(a.ck_n + c0g + lane), lin, inside, pi, pj, pk, part, lane,
+                                     ring);
     __syncwarp();
     // (b) lane l finalises shell base + l from its chunks (double-precision
     // sum of the chunk partials, each of which is exact to ~2^-48)
     const int m = base + lane;
     const bool own = m <= gend;
-    double my_dF = 0.0, g0 = 0.0;
+    int k0 = 0, nk = 0;
+    double my_dF = 0.0, nsh = 0.0;
     if (own) {
-      double t[NACC + 1];
-#pragma unroll
-      for (int v = 0; v <= NACC; v++) t[v] = 0.0;
-      const int k0 = __ldg(a.sh_c0 + m) - c0g, nk = __ldg(a.sh_nc + m);
+      k0 = __ldg(a.sh_c0 + m) - c0g;
+      nk = __ldg(a.sh_nc + m);
+      double s = 0.0;
       for (int k = k0; k < k0 + nk; k++) {
-#pragma unroll
-        for (int v = 0; v <= NACC; v++) t[v] += part[v * 32 + k];
+        s += part[k];
+        nsh += part[NACC * 32 + k];
       }
-      const double r = __ldg(rad + m);
-      const double ir = 1.0 / r;   // one division; the products differ from t / r by at most an ulp
-      const double nsh = t[NACC];
-      my_dF = nsh > 0 ? t[0] / nsh : 0.0;
-      double row[ROW];
-#pragma unroll
-      for (int v = 0; v < ROW; v++) row[v] = 0.0;
-      row[R_N] = nsh;
-#pragma unroll
-      for (int L = 0; L < 3; L++) {
-        row[R_S + L] = t[1 + L];
-        row[R_S2 + L] = t[4 + L];
-        row[R_G + L] = t[7 + L] * ir;
-        row[R_GF + L] = t[10 + L] * ir;
-      }
-      row[R_Q + 0] = (2.0 * t[13]) * ir;
-      row[R_Q + 1] = (2.0 * t[14]) * ir;
-      row[R_Q + 2] = (2.0 * t[15]) * ir;
-      row[R_Q + 3] = t[16] * ir;
-      row[R_Q + 4] = t[17] * ir;
-      row[R_Q + 5] = t[18] * ir;
-      double2* dst = reinterpret_cast<double2*>(stage + (int64_t)m * ROW);
-#pragma unroll
-      for (int v = 1; v < ROW / 2; v++) dst[v] = make_double2(row[2 * v], row[2 * v + 1]);
-      g0 = row[1];   // slots 0 (Fbar, after the scan) and 1 are stored together
+      my_dF = nsh > 0 ? s / nsh : 0.0;
     }
-    __syncwarp();
     // (c) cumulative mean overdensity (RadialShell.jl:386-390) as a scan of
     // FB[m] = r3[m] Fbar[m] = FB[m-1] + (dF[m-1] + dF[m]) / 2 * (r3[m] - r3[m-1])
     double prev_dF = __shfl_up_sync(FULL, my_dF, 1);
@@ -731,10 +743,6 @@ __device__ void gather_one(const ShellArgs& a, int64_t p, double* stage, double*
     }
     const double FBm = FB + x;
     const double fb = FBm / r3;
-    if (own) {
-      double2* dst = reinterpret_cast<double2*>(stage + (int64_t)m * ROW);
-      dst[0] = make_double2(fb, g0);
-    }
     const int last = gend - base;
     FB = __shfl_sync(FULL, FBm, last);
     dF_prev = __shfl_sync(FULL, my_dF, last);
@@ -752,11 +760,18 @@ __device__ void gather_one(const ShellArgs& a, int64_t p, double* stage, double*
         }
       }
     }
-    mdone = gend;
-    if (ADAPTIVE && mtarget < 0 && (state != 0 || mdone >= mmax)) {
+    if (ADAPTIVE && mtarget < 0 && (state != 0 || gend >= mmax)) {
       int M = max(max(m0_init, mrf), mupp_rf);
       if (state == 2) M = max(M, mcross);
       mtarget = state == 0 ? mmax : min(__ldg(a.need + M), mmax);
+      cell_lim = __ldg(a.sh_start + mtarget);
+    }
+    mdone = mtarget >= 0 ? min(gend, mtarget) : gend;
+    // (e) the rows of the group's shells up to the target; the groups after
+    // it sum the cells up to the target only (384^3: 7.1e8 -> 5.8e8 visits,
+    // 25 -> 21 M rows, 7.61 -> 7.27 ms)
+    if (m <= mdone) {
+      write_row(stage + (int64_t)m * ROW, part, k0, nk, rm, fb, nsh);
     }
     __syncwarp();
   }
@@ -856,6 +871,137 @@ __global__ void __launch_bounds__(32 * kGatherWarps, PPB_GATHER_MINB) gather_ker
   }
 }
 
+// The same for lists of one group of at most LP chunks: LP lanes per peak, 32
+// / LP peaks per warp, each step as in gather_one.  Such a peak is a few dozen
+// cells, and a warp of its own spends its time on the chain queue - geometry
+// - records - scan - pool with most lanes idle: 1.0 M peaks of 26 cells in
+// eight batches took 3.60 ms so, and take 1.06 ms.  The whole list is one
+// group, so the rows go straight to the pool.
+constexpr int LP = 8;
+template <bool COMP, bool ADAPTIVE, int SRC>
+__global__ void __launch_bounds__(32 * kGatherWarps, PPB_GATHER_MINB) gather_small_kernel(ShellArgs a) {
+  extern __shared__ double gsm[];
+  constexpr unsigned kSub = (1u << LP) - 1u;
+  constexpr int NP = 32 / LP;
+  const int lane = threadIdx.x & 31, sl = lane & (LP - 1), s0 = lane & ~(LP - 1);   // lane in the peak, its first lane
+  double* part = gsm + (size_t)(threadIdx.x >> 5) * GATHER_WARP_DOUBLES;
+  const int base = __ldg(a.grp_a), gb = __ldg(a.grp_b), c0g = __ldg(a.grp_c), ncg = __ldg(a.grp_c + 1) - c0g;
+  const int cks = sl < ncg ? __ldg(a.ck_s + c0g + sl) : 0, ckn = sl < ncg ? __ldg(a.ck_n + c0g + sl) : 0;
+  const int m = base + sl;   // the lane's shell
+  const bool has = m <= gb;
+  const int k0 = has ? __ldg(a.sh_c0 + m) - c0g + s0 : 0, nk = has ? __ldg(a.sh_nc + m) : 0;
+  const double rm = has ? __ldg(a.rad + m) : 1.0, rp = has ? __ldg(a.rad + m - 1) : 0.0;
+  const double r3 = rm * rm * rm, r3p = rp * rp * rp;
+  long long visits = 0;
+  while (true) {
+    int q = 0;
+    if (lane == 0) q = atomicAdd(a.queue, NP);
+    q = __shfl_sync(FULL, q, 0);
+    if (q >= a.npk) break;
+    q += s0 / LP;
+    bool act = q < a.npk;
+    const int64_t p = !act ? 0 : a.order ? (int64_t)__ldg(a.order + q) : (int64_t)q;
+    int4 gq = make_int4(1, 1, 1, 1), pc = make_int4(0, 0, 0, 0);
+    if (act) {
+      const float4* g2 = reinterpret_cast<const float4*>(a.geo + 2 * p);
+      float4 u, v;
+      ldg_record(g2, u, v);
+      gq = make_int4(__float_as_int(u.x), __float_as_int(u.y), __float_as_int(u.z), __float_as_int(u.w));
+      pc = make_int4(__float_as_int(v.x), __float_as_int(v.y), __float_as_int(v.z), __float_as_int(v.w));
+      if (!(pc.w & 1)) {   // invalid peak index or redshift from the caller
+        act = false;
+        if (sl == 0) {
+          atomicAdd(a.counters + CNT_BADPEAK, 1ull);
+          a.hdr[p].status = HS_BAD;
+        }
+      }
+    }
+    double fcrit = 0.0;
+    int mmax = 1;
+    float4 c0 = make_float4(0.f, 0.f, 0.f, 0.f), c1 = c0;
+    if (act) {
+      const int64_t lin = a.pk.lin[p];
+      fcrit = a.pk.fcrit[p];
+      mmax = a.mlim[p];
+      ldg_record(a.aos + 2 * lin, c0, c1);
+      if (sl < ncg && cks < __ldg(a.sh_start + mmax))
+        visits += sum_chunk<COMP, SRC>(a, c0g + sl, ckn, lin, (pc.w & 2) != 0, pc.x, pc.y, pc.z, part, lane, nullptr);
+    }
+    __syncwarp();
+    const int gend = min(gb, mmax);
+    const bool own = act && m <= gend;
+    double my_dF = 0.0, nsh = 0.0;
+    if (own) {
+      double s = 0.0;
+      for (int k = k0; k < k0 + nk; k++) {
+        s += part[k];
+        nsh += part[NACC * 32 + k];
+      }
+      my_dF = nsh > 0 ? s / nsh : 0.0;
+    }
+    double prev_dF = __shfl_up_sync(FULL, my_dF, 1, LP);
+    if (sl == 0) prev_dF = (double)c0.x;
+    double x = own ? 0.5 * (prev_dF + my_dF) * (r3 - r3p) : 0.0;
+#pragma unroll
+    for (int o = 1; o < LP; o <<= 1) {
+      const double y = __shfl_up_sync(FULL, x, o, LP);
+      if (sl >= o) x += y;
+    }
+    const double fb = x / r3;
+    // crossing (phase (d) and the inward search of gather_one)
+    const int m0_init = gq.x;
+    auto sub = [&](bool c) { return (__ballot_sync(FULL, c) >> s0) & kSub; };
+    const unsigned bi = sub(own && m == m0_init && fb < fcrit), bc = sub(own && m > m0_init && fb < fcrit),
+                   bg = sub(own && m < m0_init && fb >= fcrit);
+    int m0 = m0_init, status = HS_OK, mtarget = mmax;
+    if (bi) {
+      if (bg) m0 = base + 32 - __clz(bg);
+      else if ((double)c0.x >= fcrit) m0 = 2;
+      else status = HS_NOFCRIT;
+    } else if (bc) {
+      m0 = base + __ffs(bc) - 1;
+    }
+    if (ADAPTIVE && (bi || bc)) {
+      int M = max(max(m0_init, gq.y), gq.w);
+      if (!bi) M = max(M, m0);
+      mtarget = min(__ldg(a.need + M), mmax);
+    }
+    const int mdone = min(gend, mtarget);
+    if (status == HS_OK && m0 == 1) status = HS_M0ONE;   // zvir1p at m0 is forced to -1 < ZZon (:581-622)
+    // pool rows of the warp's peaks with one atomic
+    const int rows = act && status == HS_OK ? mdone + 1 : 0;
+    int before = 0, total = 0;
+#pragma unroll
+    for (int g = 0; g < NP; g++) {
+      const int r = __shfl_sync(FULL, rows, g * LP);
+      if (g * LP < s0) before += r;
+      total += r;
+    }
+    long long off = 0;
+    if (lane == 0 && total > 0) off = (long long)atomicAdd(a.pool_ctr, (unsigned long long)total);
+    off = __shfl_sync(FULL, off, 0) + before;
+    if (rows > 0 && off + rows > a.pool_cap) {   // the host grows the pool and runs the batch again
+      off = 0;
+      status = HS_OVERFLOW;
+    }
+    if (rows > 0 && status == HS_OK) {
+      double* dst = a.pool + off * ROW;
+      for (int v = sl; v < ROW; v += LP) dst[ROW + v] = centre_row(v, c0, c1);
+      if (own && m <= mdone) write_row(dst + (int64_t)m * ROW, part, k0, nk, rm, fb, nsh);
+    }
+    if (act && sl == 0) {
+      if (status == HS_NOFCRIT || status == HS_M0ONE)
+        atomicAdd(a.counters + (status == HS_NOFCRIT ? CNT_NOFCRIT : CNT_M0ONE), 1ull);
+      PeakHdr h;
+      h.off = rows > 0 ? off : 0; h.mdone = mdone; h.m0 = m0; h.status = status; h.pad = 0;
+      a.hdr[p] = h;
+    }
+    __syncwarp();
+  }
+  const long long tv = warp_sum_ll(visits);
+  if (lane == 0) atomicAdd(a.counters + CNT_VISITS, (unsigned long long)tv);
+}
+
 // The same with the records staged through each lane's TMA ring (tm: the
 // record array as an n^3 x 8 float tensor, box 8 x 1; n^3 < 2^31).  Shared
 // memory: the warps' rings, then their partial tables.
@@ -903,7 +1049,13 @@ __device__ __forceinline__ uint32_t spread3(uint32_t v) {
 // per-peak geometry (thread per peak) and the gather order key: the Morton
 // index of the peak's brick (2^brick_shift cells on a side, 10 bits per
 // axis), so that peaks whose spheres overlap (of any filter) are gathered
-// close in time and share cached records
+// close in time and share cached records.  The two bits above it put the
+// peaks of many cells first (a warp takes a peak whole, and one begun last
+// keeps the launch waiting): 200,000 peaks to 24 cells 5.42 -> 4.93 ms, four
+// lightcone tiles of 192^3 5.06 -> 4.89.  Not in small batches, where the
+// longest are peaks whose crossing no bound foresees, and would start later
+// (23,070 peaks of a 128^3 tile 0.26 -> 0.32 ms)
+constexpr int kLongCells = 2048, kLongPeaks = 65536;
 __global__ void geo_kernel(ShellArgs a, uint32_t* key, int32_t* idx) {
   const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= a.npk) return;
@@ -953,6 +1105,9 @@ __global__ void geo_kernel(ShellArgs a, uint32_t* key, int32_t* idx) {
     if (lin >= 0 && lin < n2 * n) {
       const int b = a.brick_shift;
       k = spread3((uint32_t)pi >> b) | (spread3((uint32_t)pj >> b) << 1) | (spread3((uint32_t)pk >> b) << 2);
+      // the cells it must at least visit, by the smallest target it can have
+      const int cells = __ldg(a.sh_start + min(__ldg(a.need + max(max(g.m0_init, g.mrf), g.mupp_rf)), mmax));
+      if (a.npk >= kLongPeaks) k |= (cells >= kLongCells ? 0u : cells >= kLongCells / 4 ? 1u : 2u) << 30;
     }
     key[p] = k;
     idx[p] = (int32_t)p;
@@ -1963,6 +2118,18 @@ void launch_shell_gather(Launch L, const ShellArgs& a, bool comp, bool adaptive,
     return;
   }
   const size_t sm = kGatherSmem;
+  if (a.ngroups == 1 && a.nck <= LP) {   // the list's chunks fit the lanes of a quarter warp
+    auto go = [&](auto c, auto ad) {
+      if (a.rec_tex) gather_small_kernel<c.value, ad.value, SRC_TEX><<<grid, block, sm, L.s>>>(a);
+      else gather_small_kernel<c.value, ad.value, SRC_LDG><<<grid, block, sm, L.s>>>(a);
+    };
+    if (comp && adaptive) go(std::true_type(), std::true_type());
+    else if (comp) go(std::true_type(), std::false_type());
+    else if (adaptive) go(std::false_type(), std::true_type());
+    else go(std::false_type(), std::false_type());
+    PPB_LAUNCHED(*L.count);
+    return;
+  }
   if (a.rec_tex) {
     if (comp && adaptive) gather_kernel<true, true, SRC_TEX><<<grid, block, sm, L.s>>>(a);
     else if (comp) gather_kernel<true, false, SRC_TEX><<<grid, block, sm, L.s>>>(a);
