@@ -8,10 +8,11 @@
 // The stage runs as four kernels on one stream:
 //
 //  gather_kernel (persistent, one warp per peak, peaks taken from a queue in
-//    list order, i.e. largest filter radius first).  A host-built schedule
-//    splits the shells (distinct r^2 of the sorted cell list; shell 1 is the
-//    peak cell) into chunks of at most 24 cells and packs 32 chunks per
-//    group, groups ending on shell boundaries.  Lane l sums chunk l of the
+//    list order or by brick; a quarter warp per peak for lists of one group of
+//    at most eight chunks).  A host-built schedule splits the shells (distinct
+//    r^2 of the sorted cell list; shell 1 is the peak cell) into chunks of at
+//    most 24 cells (16 in the first two groups) and packs 32 chunks per group,
+//    groups ending on shell boundaries.  Lane l sums chunk l of the
 //    group (four cells per step: the four cells' packed offsets in one
 //    16-byte load, four 32-byte records in flight per lane, each one 256-bit
 //    load), lane l then finalises shell l of the group from the
@@ -23,8 +24,8 @@
 //    reference forms (Float32 field times Int32 offset).  The records come
 //    through the texture pipe or as 256-bit loads (the autotuner's choice),
 //    or, as an option, through TMA-staged shared-memory rings.
-//    Adaptive truncation (optimised path): the warp stops gathering once
-//    every shell later read is in, i.e. all shells up to rad[M] + 2 with
+//    Adaptive truncation (optimised path): the warp sums and keeps only the
+//    shells that are later read, i.e. all shells up to rad[M] + 2 with
 //    M = max(crossing shell, first shell beyond ir2min, Rf window):
 //    kernel_strain's weight vanishes for |rad[mp] - rad[m1]| >= 2 and the
 //    walk only moves inward from the crossing (with no crossing at all every
@@ -33,10 +34,11 @@
 //    The kernel ends with the fcrit crossing m0 (RadialShell.jl:494-537) and
 //    moves the peak's rows from its staging slot to a pool.
 //
-//  collapse_kernel (four threads per peak).  kernel_strain windows, the
-//    inward collapse walk (four candidate steps per round), RTHL and Sbar/Srb
-//    in double precision, in the reference's summation order.  The window weights hRinteg/(u12-u0^2)^2 depend only on
-//    the radii and come from a host table.
+//  collapse kernels (1, 2, 4 or 32 threads per peak, or lane work queues).
+//    kernel_strain windows, the inward collapse walk (a candidate step per
+//    thread and round), RTHL and Sbar/Srb in double precision, in the
+//    reference's summation order.  The window weights hRinteg/(u12-u0^2)^2
+//    depend only on the radii and come from a host table.
 //
 //  zhalf_kernel (sixteen threads per collapsed peak, ten radii).  zvir_half.
 //
@@ -1115,7 +1117,7 @@ __global__ void geo_kernel(ShellArgs a, uint32_t* key, int32_t* idx) {
 }
 
 // ===========================================================================
-// collapse kernel (four threads per peak)
+// collapse kernels
 // ===========================================================================
 struct KS {
   double E[6];   // xx yy zz xy xz yz
