@@ -387,7 +387,7 @@ def run_ours(args, dist: Dist):
                          "achieved": achieved, "peak": peaks[0], "unit": "GB/s",
                          "frac": achieved / peaks[0] if peaks[0] else None,
                          "traffic": gather_traffic(last_shell_stats["visits"], last_shell_stats["pool_rows"]),
-                         "traffic_model": "dram read 2.35 B per cell visit + dram write 218 B per profile row "
+                         "traffic_model": "dram read 7.83 B per cell visit + dram write 219 B per profile row "
                                           "(ncu capture of the 384^3 launch)",
                          "peak_source": peaks[1],
                          "alg_bytes_per_launch": bytes_alg / max(1, args.steps),
@@ -407,12 +407,12 @@ def run_ours(args, dist: Dist):
 # DRAM traffic of the gather kernel: reads per cell visit (records the L2
 # does not hold) and writes per profile row (the 24-double rows of the pool
 # and the staging slots that reach DRAM), from the ncu capture of one launch
-# on the 384^3 benchmark tile (dram__bytes_read.sum 1.94 GB and
-# dram__bytes_write.sum 6.11 GB for 824,483,046 visits and 27,993,492 rows;
-# the 256^3 tile's launch, 0.403 + 1.30 GB for 179,268,416 visits and
-# 6,073,951 rows, is within 3 % of the same model)
-GATHER_DRAM_READ_PER_VISIT = 1.94e9 / 824_483_046
-GATHER_DRAM_WRITE_PER_ROW = 6.11e9 / 27_993_492
+# on the 384^3 benchmark tile (dram__bytes_read.sum 4.56 GB and
+# dram__bytes_write.sum 4.70 GB for 582,412,934 visits and 21,503,255 rows;
+# the 256^3 tile's launch, 0.918 + 1.00 GB for 126,722,480 visits and
+# 4,668,497 rows, is within 8 % of the same model)
+GATHER_DRAM_READ_PER_VISIT = 4.56e9 / 582_412_934
+GATHER_DRAM_WRITE_PER_ROW = 4.70e9 / 21_503_255
 
 
 def gather_traffic(visits: float, rows: float) -> float:
@@ -842,7 +842,7 @@ def run_shells_bench(args, dist: Dist):
             "roofline": {"kernel": "gather_kernel (compensated)", "bound": "hbm", "achieved": opt["gather_GBps"],
                          "peak": peaks[0], "unit": "GB/s", "frac": (opt["gather_GBps"] or 0) / peaks[0],
                          "traffic": gather_traffic(opt["visits"], opt["pool_rows"]), "peak_source": peaks[1],
-                         "traffic_model": "dram read 2.35 B per cell visit + dram write 218 B per profile row "
+                         "traffic_model": "dram read 7.83 B per cell visit + dram write 219 B per profile row "
                                           "(ncu capture of the 384^3 tile's launch)"},
             "optimised_over_plain": out["plain"]["shell_stage_ms"] / opt["shell_stage_ms"],
             "roofline_plain_gather": {"bound": "hbm", "achieved": out["plain"]["gather_GBps"], "peak": peaks[0],
