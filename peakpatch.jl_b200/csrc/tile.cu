@@ -653,7 +653,9 @@ int64_t peaks_phase(Run& r, TileRes& T, int n, double box, const std::vector<Win
   PPB_REQUIRE(!twin || ((size_t)(M + 4 * S) * 8 <= T.kw.bytes && (size_t)N * 4 + (size_t)(4 * S) * 8 <= T.rw.bytes),
               "twin work arrays");
   int* first = T.count.as<int>() + 2;
-  if (twin && wins.size() > 1) {
+  // window starts on the grid; one window at the origin needs none
+  const bool offset = wins.size() > 1 || wins[0].off != 0;
+  if (twin && offset) {
     std::vector<int64_t> woff;
     for (const Win& w : wins) woff.push_back(w.off);
     r.sl->woff.ensure(woff.size() * 8);
@@ -716,7 +718,7 @@ int64_t peaks_phase(Run& r, TileRes& T, int n, double box, const std::vector<Win
           launch_twin_zy(L, dkp, tw_w, cnt, T.xtw.as<float2>(), n, T.wtab.as<float>() + (size_t)f0 * 2 * qn + qn, 2 * qn,
                          (float)inv_n3, flim);
           launch_twin_rows(L, tw_w, cnt, T.xtw.as<float2>(), n, flim, nm, nm, r.fbits, f0,
-                           wins.size() > 1 ? r.sl->woff.as<int64_t>() : nullptr, first, pb);
+                           offset ? r.sl->woff.as<int64_t>() : nullptr, first, pb);
         }
       }
     });
