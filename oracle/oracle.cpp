@@ -527,7 +527,7 @@ static void dlinear_ab(const OraGrowth& G, double ai, double* Dl, double* HD, do
   if (ai > G.amin && ai < G.amax) {
     const int kk = hunt(G.a, ai);
     int nl, kkl;
-    if (kk < 2 || kk >= ntab) { nl = 2; kkl = std::max(kk - 1, 1); } else { nl = 4; kkl = kk - 2; }
+    if (kk < 2 || kk >= ntab) { nl = 2; kkl = std::max(kk - 1, 1); } else { nl = 4; kkl = std::max(kk - 2, 1); }
     const double* xa = &G.a[kkl - 1];
     const double* v1 = &G.D[kkl - 1];
     const double* v2 = &G.f[kkl - 1];

@@ -319,6 +319,7 @@ GrowthTable make_growth_table(double Om, double OB, double OL, double h) {
 
 // Dlinear_ab (Cosmology.jl:420-440 of the listing): bisection "hunt", then a
 // 4-point (2-point at the ends) Lagrange interpolation of D(a)/a and dlnD/dlna.
+// The four entries start at kk - 2, and at the first one for kk = 2.
 void dlinear_ab(const GrowthTable& G, double ai, double* Dl, double* HD, double* Da) {
   const int ntab = (int)G.a.size();
   if (ai > G.amin && ai < G.amax) {
@@ -329,7 +330,7 @@ void dlinear_ab(const GrowthTable& G, double ai, double* Dl, double* HD, double*
     }
     const int kk = jlo;
     int nl, kkl;
-    if (kk < 2 || kk >= ntab) { nl = 2; kkl = std::max(kk - 1, 1); } else { nl = 4; kkl = kk - 2; }
+    if (kk < 2 || kk >= ntab) { nl = 2; kkl = std::max(kk - 1, 1); } else { nl = 4; kkl = std::max(kk - 2, 1); }
     const double* xa = &G.a[kkl - 1];
     const double* v1 = &G.D[kkl - 1];
     const double* v2 = &G.f[kkl - 1];

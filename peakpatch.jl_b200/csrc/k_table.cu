@@ -81,7 +81,9 @@ __device__ void dlin(const TabArgs& A, double ai, double* Dl, double* HD, int* p
   const double x = ai;
   double p1 = 0.0, p2 = 0.0;
   {
-    const int k0 = four ? kk - 3 : 0;   // first of the four entries (at least four are in the table)
+    // first of the four entries (at least four are in the table): kk - 3, and
+    // entry 0 where only two lie below ai
+    const int k0 = four && kk > 2 ? kk - 3 : 0;
     const int kc = k0 + c;
     const double xc = __ldg(A.ga + kc);
     // the other three entries in ascending order

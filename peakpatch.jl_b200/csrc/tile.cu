@@ -33,7 +33,7 @@ __device__ void dlinear_ab_dev(const DevCosmo& C, double ai, double* Dl, double*
     }
     const int kk = jlo;
     int nl, kkl;
-    if (kk < 2 || kk >= ntab) { nl = 2; kkl = kk - 1 > 1 ? kk - 1 : 1; } else { nl = 4; kkl = kk - 2; }
+    if (kk < 2 || kk >= ntab) { nl = 2; kkl = kk - 1 > 1 ? kk - 1 : 1; } else { nl = 4; kkl = kk > 2 ? kk - 2 : 1; }
     const double* xa = C.ga + kkl - 1;
     const double* v1 = C.gD + kkl - 1;
     const double x = ai;
