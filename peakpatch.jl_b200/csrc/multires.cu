@@ -195,7 +195,7 @@ void mr_tile_2lpt_lap(ppb_ctx* ctx, Slot& sl, TileRes& T, int n, double box, flo
   if (lapd && fused) {
     const double dk = 2.0 * 3.141592653589793 / box;
     launch_laplacian_fused(L, T.dk.as<float2>(), T.kw.as<float2>(), T.xtw.as<float2>(), lapd, n,
-                           (float)(dk * dk * post), true);
+                           dk * dk * post, true);
   } else if (lapd) {
     const int k4[1] = {4}, z[1] = {0};
     launch_kspace(L, nullptr, T.dk.as<float2>(), T.kw.as<float2>(), Mk, n, box, k4, z, z, 1, post);

@@ -348,7 +348,7 @@ constexpr int kLpt2Arrays = 9;
 void launch_lpt2_fused(Launch L, const float2* dk, const float* delta, float2* const* w, const float2* tw, float* psi2,
                        int n, double box, bool trace);
 // irfft(|f|^2 scale dk) (one work array)
-void launch_laplacian_fused(Launch L, const float2* dk, float2* w, const float2* tw, float* out, int n, float scale,
+void launch_laplacian_fused(Launch L, const float2* dk, float2* w, const float2* tw, float* out, int n, double scale,
                             bool zero_nyq);
 // z and y transforms of the k^2-weighted twins of `cnt` <= kTwinGroup
 // consecutive filters (W_3 tables tab_stride floats apart) into w[i]

@@ -599,7 +599,7 @@ void fields_phase(Run& r, TileRes& T, int n, double box) {
   // Laplacian field (Pipeline.jl:35-51): irfft(k^2 delta_k) / n^3
   if (r.want_lap && fused) {
     const double dk = 2.0 * 3.141592653589793 / box;
-    launch_laplacian_fused(L, dkp, kw, T.xtw.as<float2>(), T.lapd.as<float>(), n, (float)(dk * dk * inv_n3 * inv_n3),
+    launch_laplacian_fused(L, dkp, kw, T.xtw.as<float2>(), T.lapd.as<float>(), n, dk * dk * inv_n3 * inv_n3,
                            false);
   } else if (r.want_lap) {
     launch_lapd(L, dkp, kw, n, box, (float)(inv_n3 * inv_n3));
