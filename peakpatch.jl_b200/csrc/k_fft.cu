@@ -629,9 +629,12 @@ void launch_laplacian_fused(Launch L, const float2* dk, float2* w, const float2*
 }
 
 int twin_flim(int n, double box, double Rf) {
-  // W_3 = k^2 exp(-(k Rf)^2 / 8): beyond k Rf = 13 the weight is below 7e-10
-  // of its values at k Rf ~ 1, under the single-precision sums' rounding
-  const double f = 13.0 * box / (6.283185307179586 * Rf);
+  // W_3 = k^2 exp(-(k Rf)^2 / 8) is largest at k Rf = sqrt(8); at 15 it is
+  // 4.6e-11 of that (at 13 3.8e-8).  The single-precision forward transform
+  // spreads a rounding of about 1e-7 of the field's rms amplitude over every
+  // mode kept; even for a field with all its power just beyond the cut that is
+  // some fifty times what the modes dropped there would add
+  const double f = 15.0 * box / (6.283185307179586 * Rf);
   return f >= n / 2 ? n / 2 : (int)f + 1;
 }
 
