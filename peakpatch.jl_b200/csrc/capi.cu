@@ -750,6 +750,7 @@ int32_t ppb_set_collapse_table(ppb_ctx* ctx, const float* tab, int32_t nx, int32
   PPB_REQUIRE(x2 > x1 && y2 > y1 && z2 > z1, "table ranges must be increasing");
   PPB_CUDA(cudaSetDevice(ctx->device));
   const size_t bytes = (size_t)nx * ny * nz * 4;
+  ctx->sh.has_tab = false;   // until the new one is in place
   ctx->sh.tab.ensure(bytes);
   PPB_CUDA(cudaMemcpy(ctx->sh.tab.p, tab, bytes, cudaMemcpyDefault));
   ctx->sh.dtab = DevTable{ctx->sh.tab.as<float>(), nullptr, nx, ny, nz, x1, x2, y1, y2, z1, z2};
@@ -769,6 +770,7 @@ int32_t ppb_set_collapse_table_f64(ppb_ctx* ctx, const double* tab, int32_t nx, 
   PPB_REQUIRE(x2 > x1 && y2 > y1 && z2 > z1, "table ranges must be increasing");
   PPB_CUDA(cudaSetDevice(ctx->device));
   const size_t bytes = (size_t)nx * ny * nz * 8;
+  ctx->sh.has_tab = false;   // until the new one is in place
   ctx->sh.tab.ensure(bytes);
   PPB_CUDA(cudaMemcpy(ctx->sh.tab.p, tab, bytes, cudaMemcpyDefault));
   ctx->sh.dtab = DevTable{nullptr, ctx->sh.tab.as<double>(), nx, ny, nz, x1, x2, y1, y2, z1, z2};
@@ -898,6 +900,7 @@ int32_t ppb_set_pk_table(ppb_ctx* ctx, const double* k, const double* pk, int32_
   }
   PPB_CUDA(cudaSetDevice(ctx->device));
   std::unique_lock<std::shared_mutex> wl(ctx->sh.mu);   // waits for runs in flight
+  ctx->sh.pk_n = 0;   // until the new table is in place
   ctx->sh.pk_lk.ensure(n * 8);
   ctx->sh.pk_lp.ensure(n * 8);
   PPB_CUDA(cudaMemcpy(ctx->sh.pk_lk.p, lk.data(), n * 8, cudaMemcpyHostToDevice));

@@ -15,7 +15,9 @@
 namespace ppb {
 
 // ---------------------------------------------------------------------------
-// error plumbing: every failing CUDA call is turned into a status + message
+// error plumbing: every failing CUDA call is turned into a status + message.
+// The runtime's record of the error is taken too: the check after the next
+// call's first launch would report it again
 // ---------------------------------------------------------------------------
 struct Error {
   int32_t code;
@@ -25,17 +27,21 @@ struct Error {
 #define PPB_CUDA(call)                                                                    \
   do {                                                                                    \
     cudaError_t e_ = (call);                                                              \
-    if (e_ != cudaSuccess)                                                                \
+    if (e_ != cudaSuccess) {                                                              \
+      cudaGetLastError();                                                                 \
       throw ::ppb::Error{e_ == cudaErrorMemoryAllocation ? PPB_ERR_NOMEM : PPB_ERR_CUDA,  \
                          std::string(#call) + ": " + cudaGetErrorString(e_)};             \
+    }                                                                                     \
   } while (0)
 
 #define PPB_CUFFT(call)                                                                   \
   do {                                                                                    \
     cufftResult r_ = (call);                                                              \
-    if (r_ != CUFFT_SUCCESS)                                                              \
+    if (r_ != CUFFT_SUCCESS) {                                                            \
+      cudaGetLastError();                                                                 \
       throw ::ppb::Error{r_ == CUFFT_ALLOC_FAILED ? PPB_ERR_NOMEM : PPB_ERR_CUDA,         \
                          std::string(#call) + ": cufft status " + std::to_string((int)r_)}; \
+    }                                                                                     \
   } while (0)
 
 #define PPB_REQUIRE(cond, msg)                                                            \

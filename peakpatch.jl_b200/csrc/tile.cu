@@ -254,9 +254,13 @@ __global__ void tile_count_kernel(const unsigned long long* keys, int npk, int s
 // plans and buffers for one grid size
 // ---------------------------------------------------------------------------
 static cufftHandle make_plan(int n, cufftType t, int batch) {
-  cufftHandle h;
+  cufftHandle h = 0;
   int dims[3] = {n, n, n};
-  PPB_CUFFT(cufftPlanMany(&h, 3, dims, nullptr, 1, 0, nullptr, 1, 0, t, batch));
+  size_t ws = 0;
+  PPB_CUFFT(cufftCreate(&h));
+  const cufftResult r = cufftMakePlanMany(h, 3, dims, nullptr, 1, 0, nullptr, 1, 0, t, batch, &ws);
+  if (r != CUFFT_SUCCESS) cufftDestroy(h);
+  PPB_CUFFT(r);
   return h;
 }
 
@@ -276,24 +280,26 @@ constexpr int kTwoStreams = 160;
 
 void TileRes::setup(int nn, cudaStream_t s, cudaStream_t s2) {
   if (n == nn) return;
+  // n says that everything below exists: taken at the end, so that a call
+  // after one that found no memory starts over
+  n = 0;
   for (cufftHandle* h : {&r2c, &c2r1, &c2r2, &c2r3, &c2r5, &c2r6, &yz1, &c2r1b, &c2r2b, &c2r3b})
     if (*h) { cufftDestroy(*h); *h = 0; }
-  n = nn;
-  const int64_t N = (int64_t)n * n * n, M = (int64_t)(n / 2 + 1) * n * n;
-  r2c = make_plan(n, CUFFT_R2C, 1);
-  c2r1 = make_plan(n, CUFFT_C2R, 1);
-  c2r3 = make_plan(n, CUFFT_C2R, 3);
-  if (!fft_supported(n)) {   // the twin's and 2LPT's full transforms
-    c2r2 = make_plan(n, CUFFT_C2R, 2);
-    c2r5 = make_plan(n, CUFFT_C2R, 5);
+  const int64_t N = (int64_t)nn * nn * nn, M = (int64_t)(nn / 2 + 1) * nn * nn;
+  r2c = make_plan(nn, CUFFT_R2C, 1);
+  c2r1 = make_plan(nn, CUFFT_C2R, 1);
+  c2r3 = make_plan(nn, CUFFT_C2R, 3);
+  if (!fft_supported(nn)) {   // the twin's and 2LPT's full transforms
+    c2r2 = make_plan(nn, CUFFT_C2R, 2);
+    c2r5 = make_plan(nn, CUFFT_C2R, 5);
   }
   for (cufftHandle h : {r2c, c2r1, c2r2, c2r3, c2r5})
     if (h) PPB_CUFFT(cufftSetStream(h, s));
 
-  if (n <= kTwoStreams) {
-    c2r1b = make_plan(n, CUFFT_C2R, 1);
-    c2r3b = make_plan(n, CUFFT_C2R, 3);
-    if (!fft_supported(n)) c2r2b = make_plan(n, CUFFT_C2R, 2);
+  if (nn <= kTwoStreams) {
+    c2r1b = make_plan(nn, CUFFT_C2R, 1);
+    c2r3b = make_plan(nn, CUFFT_C2R, 3);
+    if (!fft_supported(nn)) c2r2b = make_plan(nn, CUFFT_C2R, 2);
     for (cufftHandle h : {c2r1b, c2r2b, c2r3b})
       if (h) PPB_CUFFT(cufftSetStream(h, s2));
     kwb.ensure(3 * M * 8);
@@ -309,12 +315,13 @@ void TileRes::setup(int nn, cudaStream_t s, cudaStream_t s2) {
   rw.ensure(6 * N * 4);
   mask.ensure(N);
   count.ensure(64);
-  if (fft_supported(n)) {   // the fused transforms' twiddles and shared-memory opt-in
-    fft_prepare(n);
-    xtw.ensure((size_t)n * sizeof(float2));
+  if (fft_supported(nn)) {   // the fused transforms' twiddles and shared-memory opt-in
+    fft_prepare(nn);
+    xtw.ensure((size_t)nn * sizeof(float2));
     int64_t launched = 0;
-    launch_twiddles(Launch{s, &launched}, xtw.as<float2>(), n);
+    launch_twiddles(Launch{s, &launched}, xtw.as<float2>(), nn);
   }
+  n = nn;
 }
 
 cufftHandle TileRes::phi6(cudaStream_t s) {
@@ -346,41 +353,48 @@ void TileRes::setup_fused(cudaStream_t s) {
   if (yz1) return;
   int dims[2] = {n, n};
   const int nh = n / 2 + 1;
-  PPB_CUFFT(cufftPlanMany(&yz1, 2, dims, nullptr, 1, 0, nullptr, 1, 0, CUFFT_C2C, nh));
-  PPB_CUFFT(cufftSetStream(yz1, s));
+  size_t ws = 0;
   xpeak_prepare(n);
+  cufftHandle h = 0;
+  PPB_CUFFT(cufftCreate(&h));
+  cufftResult e = cufftMakePlanMany(h, 2, dims, nullptr, 1, 0, nullptr, 1, 0, CUFFT_C2C, nh, &ws);
+  if (e == CUFFT_SUCCESS) e = cufftSetStream(h, s);
+  if (e != CUFFT_SUCCESS) cufftDestroy(h);
+  PPB_CUFFT(e);
+  yz1 = h;
 }
 
 void TileRes::ensure_peaks(int64_t c) {
   if (c <= cap) return;
-  cap = c;
-  keys.ensure(cap * 8);
-  vals.ensure(cap * 4);
-  ff.ensure(cap * 4);
-  lap.ensure(cap * 4);
-  keys_s.ensure(cap * 8);
-  vals_s.ensure(cap * 4);
-  p_lin.ensure(cap * 8);
-  p_Rf.ensure(cap * 8);
-  p_ir2.ensure(cap * 4);
-  p_np.ensure(cap * 4);
-  p_Z.ensure(cap * 8);
-  p_fc.ensure(cap * 8);
-  p_FcRf.ensure(cap * 4);
-  p_d2Rf.ensure(cap * 4);
-  p_pos.ensure(cap * 24);
-  res.ensure(cap * RES_N * 8);
-  flags.ensure(cap * 4 + 4);
-  offs.ensure(cap * 4 + 4);
-  rec.ensure(cap * 33 * 4);
-  rthl.ensure(cap * 4);
+  cap = 0;   // until every buffer has the new size
+  keys.ensure(c * 8);
+  vals.ensure(c * 4);
+  ff.ensure(c * 4);
+  lap.ensure(c * 4);
+  keys_s.ensure(c * 8);
+  vals_s.ensure(c * 4);
+  p_lin.ensure(c * 8);
+  p_Rf.ensure(c * 8);
+  p_ir2.ensure(c * 4);
+  p_np.ensure(c * 4);
+  p_Z.ensure(c * 8);
+  p_fc.ensure(c * 8);
+  p_FcRf.ensure(c * 4);
+  p_d2Rf.ensure(c * 4);
+  p_pos.ensure(c * 24);
+  res.ensure(c * RES_N * 8);
+  flags.ensure(c * 4 + 4);
+  offs.ensure(c * 4 + 4);
+  rec.ensure(c * 33 * 4);
+  rthl.ensure(c * 4);
   size_t t1 = 0, t2 = 0;
   PPB_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, t1, keys.as<unsigned long long>(), keys_s.as<unsigned long long>(),
-                                           vals.as<uint32_t>(), vals_s.as<uint32_t>(), (int)cap, 0, 64));
-  PPB_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, t2, flags.as<int>(), offs.as<int>(), (int)cap + 1));
+                                           vals.as<uint32_t>(), vals_s.as<uint32_t>(), (int)c, 0, 64));
+  PPB_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, t2, flags.as<int>(), offs.as<int>(), (int)c + 1));
   size_t t3 = 0;
-  PPB_CUDA(cub::DeviceReduce::Max(nullptr, t3, rthl.as<float>(), rthl.as<float>(), (int)cap));
+  PPB_CUDA(cub::DeviceReduce::Max(nullptr, t3, rthl.as<float>(), rthl.as<float>(), (int)c));
   tmp.ensure(std::max(std::max(t1, t2), t3) + 256);
+  cap = c;
 }
 
 // ---------------------------------------------------------------------------
