@@ -23,6 +23,9 @@ struct TileRes {
   // (0 where one stream is used)
   cufftHandle c2r1b = 0, c2r2b = 0, c2r3b = 0;
   DevBuf kwb, rwb;
+  // one work area for the plans of each stream, which run one after another
+  DevBuf ws, wsb;
+  void share_work(size_t need, size_t need_b);
   // in-place inverse C2C of contiguous n x n (kz, ky) planes, batched over
   // the n/2+1 kx: the filter bank's transforms before the fused x pass (0
   // where unsupported)

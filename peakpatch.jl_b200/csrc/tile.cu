@@ -13,6 +13,8 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <map>
+#include <mutex>
 
 #include "ppb_ctx.h"
 
@@ -253,15 +255,30 @@ __global__ void tile_count_kernel(const unsigned long long* keys, int npk, int s
 // ---------------------------------------------------------------------------
 // plans and buffers for one grid size
 // ---------------------------------------------------------------------------
-static cufftHandle make_plan(int n, cufftType t, int batch) {
+// a plan on stream s whose work area is set by share_work; ws: the largest
+// one needed
+static cufftHandle make_plan(int rank, int n, cufftType t, int batch, cudaStream_t s, size_t& ws) {
   cufftHandle h = 0;
   int dims[3] = {n, n, n};
-  size_t ws = 0;
+  size_t w = 0;
   PPB_CUFFT(cufftCreate(&h));
-  const cufftResult r = cufftMakePlanMany(h, 3, dims, nullptr, 1, 0, nullptr, 1, 0, t, batch, &ws);
-  if (r != CUFFT_SUCCESS) cufftDestroy(h);
-  PPB_CUFFT(r);
+  cufftResult e = cufftSetAutoAllocation(h, 0);
+  if (e == CUFFT_SUCCESS) e = cufftMakePlanMany(h, rank, dims, nullptr, 1, 0, nullptr, 1, 0, t, batch, &w);
+  if (e == CUFFT_SUCCESS) e = cufftSetStream(h, s);
+  if (e != CUFFT_SUCCESS) cufftDestroy(h);
+  PPB_CUFFT(e);
+  ws = std::max(ws, w);
   return h;
+}
+
+void TileRes::share_work(size_t need, size_t need_b) {
+  ws.ensure(std::max<size_t>(need, 256));
+  for (cufftHandle h : {r2c, c2r1, c2r2, c2r3, c2r5, c2r6, yz1})
+    if (h) PPB_CUFFT(cufftSetWorkArea(h, ws.p));
+  if (!c2r1b) return;
+  wsb.ensure(std::max<size_t>(need_b, 256));
+  for (cufftHandle h : {c2r1b, c2r2b, c2r3b})
+    if (h) PPB_CUFFT(cufftSetWorkArea(h, wsb.p));
 }
 
 TileRes::~TileRes() {
@@ -278,6 +295,9 @@ TileRes::~TileRes() {
 // 1.87); the kernels of a 192^3 field fill it
 constexpr int kTwoStreams = 160;
 
+// the second stream's smoothed field, and its full twin where there is one
+static uint64_t second_field_bytes(uint64_t n) { return n * n * n * (fft_supported((int)n) ? 4 : 8); }
+
 void TileRes::setup(int nn, cudaStream_t s, cudaStream_t s2) {
   if (n == nn) return;
   // n says that everything below exists: taken at the end, so that a call
@@ -286,25 +306,22 @@ void TileRes::setup(int nn, cudaStream_t s, cudaStream_t s2) {
   for (cufftHandle* h : {&r2c, &c2r1, &c2r2, &c2r3, &c2r5, &c2r6, &yz1, &c2r1b, &c2r2b, &c2r3b})
     if (*h) { cufftDestroy(*h); *h = 0; }
   const int64_t N = (int64_t)nn * nn * nn, M = (int64_t)(nn / 2 + 1) * nn * nn;
-  r2c = make_plan(nn, CUFFT_R2C, 1);
-  c2r1 = make_plan(nn, CUFFT_C2R, 1);
-  c2r3 = make_plan(nn, CUFFT_C2R, 3);
+  size_t w = 0, wb = 0;
+  r2c = make_plan(3, nn, CUFFT_R2C, 1, s, w);
+  c2r1 = make_plan(3, nn, CUFFT_C2R, 1, s, w);
+  c2r3 = make_plan(3, nn, CUFFT_C2R, 3, s, w);
   if (!fft_supported(nn)) {   // the twin's and 2LPT's full transforms
-    c2r2 = make_plan(nn, CUFFT_C2R, 2);
-    c2r5 = make_plan(nn, CUFFT_C2R, 5);
+    c2r2 = make_plan(3, nn, CUFFT_C2R, 2, s, w);
+    c2r5 = make_plan(3, nn, CUFFT_C2R, 5, s, w);
   }
-  for (cufftHandle h : {r2c, c2r1, c2r2, c2r3, c2r5})
-    if (h) PPB_CUFFT(cufftSetStream(h, s));
-
   if (nn <= kTwoStreams) {
-    c2r1b = make_plan(nn, CUFFT_C2R, 1);
-    c2r3b = make_plan(nn, CUFFT_C2R, 3);
-    if (!fft_supported(nn)) c2r2b = make_plan(nn, CUFFT_C2R, 2);
-    for (cufftHandle h : {c2r1b, c2r2b, c2r3b})
-      if (h) PPB_CUFFT(cufftSetStream(h, s2));
+    c2r1b = make_plan(3, nn, CUFFT_C2R, 1, s2, wb);
+    c2r3b = make_plan(3, nn, CUFFT_C2R, 3, s2, wb);
+    if (!fft_supported(nn)) c2r2b = make_plan(3, nn, CUFFT_C2R, 2, s2, wb);
     kwb.ensure(3 * M * 8);
-    rwb.ensure(2 * N * 4);
+    rwb.ensure(second_field_bytes(nn));
   }
+  share_work(w, wb);
 
   delta.ensure(N * 4);
   dk.ensure(M * 8);
@@ -326,15 +343,17 @@ void TileRes::setup(int nn, cudaStream_t s, cudaStream_t s2) {
 
 cufftHandle TileRes::phi6(cudaStream_t s) {
   if (!c2r6) {
-    c2r6 = make_plan(n, CUFFT_C2R, 6);
-    PPB_CUFFT(cufftSetStream(c2r6, s));
+    size_t w = ws.bytes;
+    PPB_CUDA(cudaStreamSynchronize(s));   // the work area may move
+    c2r6 = make_plan(3, n, CUFFT_C2R, 6, s, w);
+    share_work(w, wsb.bytes);
   }
   return c2r6;
 }
 
 size_t TileRes::bytes() const {
   size_t b = 0;
-  for (const DevBuf* d : {&delta, &dk, &psi, &psi2, &lapd, &aos, &kw, &rw, &kwb, &rwb, &mask, &count, &wtab, &keys, &vals, &ff,
+  for (const DevBuf* d : {&delta, &dk, &psi, &psi2, &lapd, &aos, &kw, &rw, &kwb, &rwb, &ws, &wsb, &mask, &count, &wtab, &keys, &vals, &ff,
                           &lap, &keys_s, &vals_s, &tmp, &p_lin, &p_Rf, &p_ir2, &p_np, &p_Z, &p_fc, &p_FcRf, &p_d2Rf,
                           &p_pos, &res, &flags, &offs, &rec, &rthl, &xtw})
     b += d->bytes;
@@ -351,17 +370,11 @@ void fft_work_arrays(TileRes& T, int n, float2** w) {
 
 void TileRes::setup_fused(cudaStream_t s) {
   if (yz1) return;
-  int dims[2] = {n, n};
-  const int nh = n / 2 + 1;
-  size_t ws = 0;
   xpeak_prepare(n);
-  cufftHandle h = 0;
-  PPB_CUFFT(cufftCreate(&h));
-  cufftResult e = cufftMakePlanMany(h, 2, dims, nullptr, 1, 0, nullptr, 1, 0, CUFFT_C2C, nh, &ws);
-  if (e == CUFFT_SUCCESS) e = cufftSetStream(h, s);
-  if (e != CUFFT_SUCCESS) cufftDestroy(h);
-  PPB_CUFFT(e);
-  yz1 = h;
+  size_t w = ws.bytes;
+  PPB_CUDA(cudaStreamSynchronize(s));   // the work area may move
+  yz1 = make_plan(2, n, CUFFT_C2C, n / 2 + 1, s, w);
+  share_work(w, wsb.bytes);
 }
 
 void TileRes::ensure_peaks(int64_t c) {
@@ -423,13 +436,39 @@ uint64_t tile_footprint(const ppb_tile_params* p) { return tile_bytes_estimate(p
 // waits for all slots' work on the device).  A larger count still grows them.
 int64_t initial_peak_capacity(int64_t N) { return std::max<int64_t>(1 << 16, std::min<int64_t>(N / 40, 1 << 22)); }
 
+// work areas of both streams' plans of an n <= kTwoStreams grid, as the
+// library states them before a plan is made (about 1 ms a plan, so kept by n)
+static uint64_t plan_work_bytes(int n) {
+  static std::mutex mu;
+  static std::map<int, uint64_t> known;
+  std::lock_guard<std::mutex> lk(mu);
+  auto it = known.find(n);
+  if (it != known.end()) return it->second;
+  auto work = [&](cufftType t, int batch) {
+    int dims[3] = {n, n, n};
+    size_t w = 0;
+    const cufftResult r = cufftEstimateMany(3, dims, nullptr, 1, 0, nullptr, 1, 0, t, batch, &w);
+    if (r == CUFFT_SUCCESS) return (uint64_t)w;
+    return (uint64_t)(batch + 1) * 16 * (n / 2 + 1) * n * n;   // the most of any size: two half spectra per transform and two more
+  };
+  const uint64_t two = std::max(work(CUFFT_C2R, 1), work(CUFFT_C2R, 3));
+  uint64_t one = std::max(two, work(CUFFT_R2C, 1));
+  if (!fft_supported(n)) one = std::max(one, work(CUFFT_C2R, 5));
+  return known[n] = one + two;
+}
+
 uint64_t tile_bytes_estimate(int nn) {
   const uint64_t n = (uint64_t)nn, N = n * n * n, M = (n / 2 + 1) * n * n;
   // TileRes fields: delta, psi (3), psi2 (3), lapd, rw (6), mask, aos (8 floats), dk + kw (7 complex)
   const uint64_t fields = N * 4 * (1 + 3 + 3 + 1 + 6) + N + N * 32 + M * 8 * 7;
   // peak, result and record buffers: initial_peak_capacity (1/40 peak per
-  // cell), 0.5 KB each; plans and their work areas
-  return fields + N * 13 + ((uint64_t)64 << 20);
+  // cell), 0.5 KB each; plans
+  uint64_t b = fields + N * 13 + ((uint64_t)64 << 20);
+  // small grids: the second stream's buffers, and the work areas of both
+  // streams' plans, most of what such a size holds beyond its fields
+  // (142^3: 0.13 GB of 0.59)
+  if (nn <= kTwoStreams) b += M * 24 + second_field_bytes(n) + plan_work_bytes(nn);
+  return b;
 }
 
 uint64_t shell_bytes_estimate(int nn) {
