@@ -91,8 +91,23 @@ cudaTextureObject_t Slot::record_texture(const float4* aos, int n) {
 
 // the record array of a stub call may be among them: its texture goes first
 void Slot::release_stub() {
-  drop_record_texture();
-  for (DevBuf& b : stub) b.release();
+  for (DevBuf& b : stub) {
+    if (b.p && b.p == rec_ptr) drop_record_texture();
+    b.release();
+  }
+}
+
+size_t Slot::stub_bytes() const {
+  size_t b = 0;
+  for (const DevBuf& d : stub) b += d.bytes;
+  return b;
+}
+
+bool Slot::give_back_stub() {
+  if (stub_busy || stub_bytes() == 0) return false;
+  PPB_CUDA(cudaStreamSynchronize(stream));
+  release_stub();
+  return true;
 }
 
 void Slot::release_buffers() {
@@ -122,7 +137,7 @@ size_t Slot::shell_bytes() const {
                           &okey, &okey2, &oidx, &oidx2, &otmp, &tcen, &tcount, &t_aos, &t_lapd, &woff, &mlim, &anchors, &mr_in,
                           &mr_out, &mr_aux, &mr_rec, &mr_axis, &mr_amp, &pft})
     b += d->bytes;
-  for (const DevBuf& d : stub) b += d.bytes;
+  b += stub_bytes();
   if (iso) b += iso->bytes();
   return b;
 }
@@ -147,10 +162,11 @@ TileRes& Slot::tile_for(int n) {
   auto it = tiles.find(n);
   if (it == tiles.end()) {
     while ((int)tiles.size() >= std::max(1, max_tiles)) drop_tile(lru_tile(n));
-    if (!tiles.empty()) {   // room for the new size's buffers, else give up older sizes
+    if (!tiles.empty() || stub_bytes() > 0) {   // room for the new size's buffers, else give up stub buffers, older sizes
       const uint64_t need = tile_bytes_estimate(n);
       size_t fr = 0, tot = 0;
       PPB_CUDA(cudaMemGetInfo(&fr, &tot));
+      if ((uint64_t)fr < need + need / 4 && give_back_stub()) PPB_CUDA(cudaMemGetInfo(&fr, &tot));
       while (!tiles.empty() && (uint64_t)fr < need + need / 4) {
         drop_tile(lru_tile(n));
         PPB_CUDA(cudaMemGetInfo(&fr, &tot));
@@ -528,10 +544,12 @@ void ppb_ctx::run_shells(Slot& sl, ShellArgs& a, bool comp, bool adaptive, Shell
   auto set_budget = [&](double peaks) {
     budget_rows = (int64_t)(sl.pool.bytes / row_bytes);
     if (peaks * rpp * 1.25 + 4096 <= (double)budget_rows) return;
-    size_t fr = 0, tot = 0;
-    PPB_CUDA(cudaMemGetInfo(&fr, &tot));
-    budget_rows = std::max<int64_t>(
-        1 << 16, (int64_t)(std::min<size_t>((size_t)32 << 30, (fr + sl.pool.bytes) / 2) / row_bytes));
+    do {
+      size_t fr = 0, tot = 0;
+      PPB_CUDA(cudaMemGetInfo(&fr, &tot));
+      budget_rows = std::max<int64_t>(
+          1 << 16, (int64_t)(std::min<size_t>((size_t)32 << 30, (fr + sl.pool.bytes) / 2) / row_bytes));
+    } while (peaks * rpp * 1.25 + 4096 > (double)budget_rows && sl.give_back_stub());
   };
   set_budget((double)a.npk);
   ShellStats s{};
@@ -804,9 +822,11 @@ int32_t ppb_make_collapse_table(ppb_ctx* ctx, const ppb_table_params* p, double*
   for (int i = 0; i < p->Nx; i++) F[i] = std::pow(10.0, p->X1 + i * dX);
   const int64_t nn = (int64_t)p->Nx * p->Ny * p->Nz;
   DevBuf dF, dout, dsteps;
-  dF.ensure(F.size() * 8);
-  dout.ensure((size_t)nn * 8);
-  dsteps.ensure(8);
+  sl.with_room([&] {
+    dF.ensure(F.size() * 8);
+    dout.ensure((size_t)nn * 8);
+    dsteps.ensure(8);
+  });
   PPB_CUDA(cudaMemcpyAsync(dF.p, F.data(), F.size() * 8, cudaMemcpyHostToDevice, sl.stream));
   PPB_CUDA(cudaMemsetAsync(dsteps.p, 0, 8, sl.stream));
   PPB_CUDA(cudaEventRecord(sl.stage_ev[0], sl.stream));
@@ -851,7 +871,7 @@ int32_t ppb_generate_fields(ppb_ctx* ctx, const ppb_tile_params* p, float* delta
   PPB_CUDA(cudaSetDevice(ctx->device));
   PPB_REQUIRE(p != nullptr, "params is null");
   std::shared_lock<std::shared_mutex> rl(ctx->sh.mu);
-  generate_fields_core(ctx, ctx->sync, p, delta, psi, psi2, lapd);
+  ctx->sync.with_room([&] { generate_fields_core(ctx, ctx->sync, p, delta, psi, psi2, lapd); });
   return PPB_OK;
   PPB_GUARD_END(ctx)
 }
@@ -880,8 +900,10 @@ int32_t ppb_peak_find_tile(ppb_ctx* ctx, const float* delta_tile, int32_t n, con
   o.d2Rf = d2Rf;
   o.filter = filter;
   o.npeaks = npeaks;
-  peak_find_tile_core(ctx, ctx->sync, delta_tile, n, Rf, fcrit, nfilt, mask, xbx, ybx, zbx, alatt, nbuff, wsmooth,
-                      ioutshear, o);
+  ctx->sync.with_room([&] {
+    peak_find_tile_core(ctx, ctx->sync, delta_tile, n, Rf, fcrit, nfilt, mask, xbx, ybx, zbx, alatt, nbuff, wsmooth,
+                        ioutshear, o);
+  });
   return PPB_OK;
   PPB_GUARD_END(ctx)
 }
@@ -924,7 +946,7 @@ int32_t ppb_run_tile_timed(ppb_ctx* ctx, const ppb_tile_params* p, const double*
   PPB_REQUIRE(out != nullptr, "output buffer is null");
   std::shared_lock<std::shared_mutex> rl(ctx->sh.mu);
   TileOut o;
-  run_tile_core(ctx, ctx->sync, p, Rf, nfilt, &o);
+  ctx->sync.with_room([&] { run_tile_core(ctx, ctx->sync, p, Rf, nfilt, &o); });
   out->nfields = o.nfields;
   out->count = o.count;
   out->npeaks = o.npeaks;
@@ -949,7 +971,7 @@ int32_t ppb_run_multitile(ppb_ctx* ctx, const ppb_tile_params* p, const double* 
   PPB_REQUIRE(ntiles >= 0 && (ntiles == 0 || tiles != nullptr), "tiles must hold ntiles triples");
   std::shared_lock<std::shared_mutex> rl(ctx->sh.mu);
   TileOut o;
-  run_multitile_core(ctx, ctx->sync, p, Rf, nfilt, ntile, tiles, ntiles, &o);
+  ctx->sync.with_room([&] { run_multitile_core(ctx, ctx->sync, p, Rf, nfilt, ntile, tiles, ntiles, &o); });
   out->nfields = o.nfields;
   out->count = o.count;
   out->npeaks = o.npeaks;
@@ -974,7 +996,9 @@ int32_t ppb_run_multitile_split(ppb_ctx* ctx, const ppb_tile_params* p, const do
   PPB_REQUIRE(ntiles >= 0 && (ntiles == 0 || tiles != nullptr), "tiles must hold ntiles triples");
   std::shared_lock<std::shared_mutex> rl(ctx->sh.mu);
   TileOut o;
-  run_multitile_split_core(ctx, ctx->sync, p, Rf, nfilt, ntile, coarse_factor, coarse_grid, tiles, ntiles, &o);
+  ctx->sync.with_room([&] {
+    run_multitile_split_core(ctx, ctx->sync, p, Rf, nfilt, ntile, coarse_factor, coarse_grid, tiles, ntiles, &o);
+  });
   out->nfields = o.nfields;
   out->count = o.count;
   out->npeaks = o.npeaks;
@@ -1005,13 +1029,16 @@ int32_t ppb_merge_catalog(ppb_ctx* ctx, const float* records, int64_t n, int32_t
   if (n == 0) return PPB_OK;
   Slot& sl = ctx->sync;
   const size_t bytes = (size_t)n * nfields * 4;
-  const float* d_rec = (const float*)stage_in(sl.merge.in, records, bytes, sl.stream);
   float* d_out = out;
-  if (!is_device_ptr(out)) {
-    sl.merge.out.ensure(bytes);
-    d_out = sl.merge.out.as<float>();
-  }
-  const int64_t m = merge_catalog_device(sl, d_rec, n, nfields, d_out);
+  int64_t m = 0;
+  sl.with_room([&] {
+    const float* d_rec = (const float*)stage_in(sl.merge.in, records, bytes, sl.stream);
+    if (!is_device_ptr(out)) {
+      sl.merge.out.ensure(bytes);
+      d_out = sl.merge.out.as<float>();
+    }
+    m = merge_catalog_device(sl, d_rec, n, nfields, d_out);
+  });
   if (m > 0 && d_out != out) copy_out(out, d_out, (size_t)m * nfields * 4, sl.stream);
   PPB_CUDA(cudaStreamSynchronize(sl.stream));
   *n_out = m;
@@ -1062,7 +1089,7 @@ int32_t ppb_noise_threefry(ppb_ctx* ctx, float* out, int32_t n, uint64_t seed) {
     PPB_CUDA(cudaStreamSynchronize(sl.stream));
   } else {
     DevBuf tmp;
-    tmp.ensure(bytes);
+    sl.with_room([&] { tmp.ensure(bytes); });
     launch_noise(Launch{sl.stream, &sl.launches}, tmp.as<float>(), n, seed);
     copy_out(out, tmp.p, bytes, sl.stream);
   }
@@ -1091,7 +1118,14 @@ int32_t ppb_alloc_device(ppb_ctx* ctx, size_t bytes, void** out) {
   if (!ctx || !out || bytes == 0) return PPB_ERR_INVALID;
   PPB_GUARD_BEGIN
   PPB_CUDA(cudaSetDevice(ctx->device));
-  PPB_CUDA(cudaMalloc(out, bytes));
+  const auto alloc = [&] { PPB_CUDA(cudaMalloc(out, bytes)); };
+  try {
+    alloc();
+  } catch (const ppb::Error&) {
+    std::lock_guard<std::recursive_mutex> lk(ctx->mu);
+    if (!ctx->sync.give_back_stub()) throw;
+    alloc();
+  }
   return PPB_OK;
   PPB_GUARD_END(ctx)
 }

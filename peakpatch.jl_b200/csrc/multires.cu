@@ -309,7 +309,7 @@ int32_t guarded(ppb_ctx* ctx, F&& body) {
   std::lock_guard<std::recursive_mutex> lk(ctx->mu);
   try {
     PPB_CUDA(cudaSetDevice(ctx->device));
-    body();
+    ctx->sync.with_room(body);   // results are copied out last
     return PPB_OK;
   } catch (const ppb::Error& e) {
     ctx->set_error(e.msg);

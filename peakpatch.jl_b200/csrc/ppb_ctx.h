@@ -146,7 +146,22 @@ struct Slot {
   DevBuf mr_in, mr_out, mr_aux, mr_rec;             // multi-resolution: staged inputs, outputs, records
   DevBuf mr_axis, mr_amp;                           // multi-resolution: tricubic axis tables, coarse amplitudes
   DevBuf stub[19];                                  // the stub entry points' staging and outputs (stubs.cu)
+  bool stub_busy = false;                           // a stub call is using them
+  size_t stub_bytes() const;
   void release_stub();
+  // where memory is short: the kept stub buffers are freed (false: none, or
+  // in use).  with_room runs f, and once more if it found no memory while
+  // they were held; f must not have changed what the caller gave it
+  bool give_back_stub();
+  template <class F> void with_room(F&& f) {
+    try {
+      f();
+      return;
+    } catch (const Error& e) {
+      if (e.code != PPB_ERR_NOMEM || !give_back_stub()) throw;
+    }
+    f();
+  }
   DevBuf pft;                                       // ppb_peak_find_tile: unpacked (i, j, k), ipp, filter
   int gather_bps[2][2][2] = {};                      // gather blocks per SM by [comp][adaptive][ring]
   double rows_per_peak[2] = {0.0, 0.0};             // pool rows per peak seen last, by adaptive

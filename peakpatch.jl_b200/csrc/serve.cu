@@ -168,7 +168,17 @@ void Server::worker_loop(SlotState* st) {
     TileOut o;
     try {
       std::shared_lock<std::shared_mutex> rl(ctx->sh.mu);
-      run_tile_core(ctx, *st->slot, &r->p, r->Rf.data(), (int)r->Rf.size(), &o);
+      try {
+        run_tile_core(ctx, *st->slot, &r->p, r->Rf.data(), (int)r->Rf.size(), &o);
+      } catch (const Error& e) {
+        // no memory: once more without the synchronous slot's kept stub
+        // buffers, unless a call on that slot is running (never waited for:
+        // it may wait for this run to end)
+        std::unique_lock<std::recursive_mutex> lk(ctx->mu, std::try_to_lock);
+        if (e.code != PPB_ERR_NOMEM || !lk || !ctx->sync.give_back_stub()) throw;
+        lk.unlock();
+        run_tile_core(ctx, *st->slot, &r->p, r->Rf.data(), (int)r->Rf.size(), &o);
+      }
       r->rec.resize((size_t)o.count * o.nfields);
       if (o.count > 0) copy_out(r->rec.data(), o.d_records, r->rec.size() * sizeof(float), st->slot->stream);
     } catch (const Error& e) {

@@ -84,16 +84,22 @@ __global__ void skip_out_kernel(const int32_t* skip, int64_t nq, double* out) {
 // and the call has waited for the stream when it ends without an error.
 struct StubCall {
   Slot& sl;
-  explicit StubCall(Slot& s) : sl(s) {}
+  explicit StubCall(Slot& s) : sl(s) { sl.stub_busy = true; }
   DevBuf& operator[](int i) { return sl.stub[i]; }
   ~StubCall() {
-    size_t b = 0;
-    for (const DevBuf& d : sl.stub) b += d.bytes;
-    if (b <= kStubKeep) return;
+    sl.stub_busy = false;
+    if (sl.stub_bytes() <= kStubKeep) return;
     cudaStreamSynchronize(sl.stream);
     sl.release_stub();
   }
 };
+
+// a call that found no memory while it or another one's kept buffers were
+// held may be repeated without them: they are freed, and only the first
+// attempt starts with any (kept: bytes at its start)
+bool without_kept(ppb_ctx* ctx, const Error& e, size_t kept) {
+  return e.code == PPB_ERR_NOMEM && kept > 0 && ctx->sync.give_back_stub();
+}
 
 }  // namespace
 
@@ -104,6 +110,8 @@ int32_t ppb_find_peaks(ppb_ctx* ctx, const float* delta, int8_t* mask, int32_t n
                        int64_t* ipp, float* pdelta, int64_t* npeaks) {
   if (!ctx) return PPB_ERR_INVALID;
   std::lock_guard<std::recursive_mutex> lk(ctx->mu);
+  const size_t kept = ctx->sync.stub_bytes();
+  bool marked = false;   // the caller's device mask may have been written
   try {
     PPB_REQUIRE(delta && mask && pi && pj && pk && ipp && pdelta && npeaks, "null argument");
     PPB_REQUIRE(n1 >= 3 && n2 >= 3 && n3 >= 3 && nbuff >= 1, "grid must be >= 3 cells with nbuff >= 1");
@@ -141,6 +149,7 @@ int32_t ppb_find_peaks(ppb_ctx* ctx, const float* delta, int8_t* mask, int32_t n
     // the lapd sample slot aliases ff; nothing reads it here
     lapdummy.ensure(cap * 4);
     pb.lap = lapdummy.as<float>();
+    marked = mask_dev;
     launch_peakfind(Launch{s, &ctx->sync.launches}, dd, nullptr, dm, n1, n2, n3, n1, (int64_t)n1 * n2, nbuff, fcrit,
                     0ull, pb);
     int c = 0;
@@ -185,6 +194,8 @@ int32_t ppb_find_peaks(ppb_ctx* ctx, const float* delta, int8_t* mask, int32_t n
     *npeaks = np;
     return PPB_OK;
   } catch (const ppb::Error& e) {
+    if (!marked && without_kept(ctx, e, kept))
+      return ppb_find_peaks(ctx, delta, mask, n1, n2, n3, nbuff, fcrit, max_peaks, pi, pj, pk, ipp, pdelta, npeaks);
     ctx->set_error(e.msg);
     return e.code;
   } catch (...) {
@@ -200,6 +211,7 @@ static int32_t analyse_peaks_impl(ppb_ctx* ctx, const float* delta, const float*
                                   const int32_t* r2lim, double alatt, int32_t plain, double* out) {
   if (!ctx) return PPB_ERR_INVALID;
   std::lock_guard<std::recursive_mutex> lk(ctx->mu);
+  const size_t kept = ctx->sync.stub_bytes();
   try {
     PPB_REQUIRE(delta && etax && etay && etaz && ipp && Rf && ir2min && ZZon && fcrit && out, "null argument");
     PPB_REQUIRE((eta2x == nullptr) == (eta2y == nullptr) && (eta2y == nullptr) == (eta2z == nullptr),
@@ -270,6 +282,9 @@ static int32_t analyse_peaks_impl(ppb_ctx* ctx, const float* delta, const float*
     PPB_CUDA(cudaStreamSynchronize(s));
     return PPB_OK;
   } catch (const ppb::Error& e) {
+    if (without_kept(ctx, e, kept))
+      return analyse_peaks_impl(ctx, delta, etax, etay, etaz, eta2x, eta2y, eta2z, lapd, n, nhunt, npk, ipp, Rf, ir2min,
+                                ZZon, fcrit, r2lim, alatt, plain, out);
     ctx->set_error(e.msg);
     return e.code;
   } catch (...) {
@@ -305,6 +320,7 @@ int32_t ppb_analyse_peaks_multirf(ppb_ctx* ctx, const float* delta, const float*
                                   int32_t plain, double* out) {
   if (!ctx) return PPB_ERR_INVALID;
   std::lock_guard<std::recursive_mutex> lk(ctx->mu);
+  const size_t kept = ctx->sync.stub_bytes();
   try {
     PPB_REQUIRE(delta && etax && etay && etaz && boff && pi && pj && pk && Rf && ir2min && out, "null argument");
     PPB_REQUIRE((eta2x == nullptr) == (eta2y == nullptr) && (eta2y == nullptr) == (eta2z == nullptr),
@@ -419,6 +435,10 @@ int32_t ppb_analyse_peaks_multirf(ppb_ctx* ctx, const float* delta, const float*
     PPB_CUDA(cudaStreamSynchronize(s));
     return PPB_OK;
   } catch (const ppb::Error& e) {
+    if (without_kept(ctx, e, kept))
+      return ppb_analyse_peaks_multirf(ctx, delta, etax, etay, etaz, eta2x, eta2y, eta2z, lapd, n, nhunt, nbatch, boff,
+                                       pi, pj, pk, Rf, ir2min, ZZon_pp, fcrit_pp, ZZon, fcrit, alatt, mask, nbuff,
+                                       rmax2rs, plain, out);
     ctx->set_error(e.msg);
     return e.code;
   } catch (...) {
