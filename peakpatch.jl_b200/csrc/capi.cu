@@ -532,11 +532,12 @@ void ppb_ctx::run_shells(Slot& sl, ShellArgs& a, bool comp, bool adaptive, Shell
   sl.anchors.ensure(std::max<size_t>(1, (size_t)a.nck) * kAnchorStride * sizeof(float2));
   a.ck_K = sl.anchors.as<float2>();
   PPB_CUDA(cudaMemsetAsync(sl.counters.p, 0, 16 * 8, stream));
-  // profile pool: sized from the rows per peak of the previous call; peaks
-  // run in batches that fit the pool budget, and a batch whose rows overflow
-  // the pool runs again with a larger pool or fewer peaks
+  // profile pool: sized from the rows per peak of the previous batch, for the
+  // first one from the previous call; peaks run in batches that fit the pool
+  // budget, and a batch whose rows overflow the pool runs again with a larger
+  // pool or fewer peaks
   const size_t row_bytes = ROW * sizeof(double);
-  double& rpp = sl.rows_per_peak[adaptive];
+  double rpp = sl.rows_per_peak[adaptive], most = 0.0;
   if (rpp <= 0.0) rpp = adaptive ? 64.0 : (double)(a.mmax + 1);
   // pool budget: half of the free memory (with the pool's own), at most 32 GB;
   // the free-memory query runs only when the pool would have to grow
@@ -667,15 +668,18 @@ void ppb_ctx::run_shells(Slot& sl, ShellArgs& a, bool comp, bool adaptive, Shell
     s.ms += k[0] + k[1] + k[2] + k[3];
     s.pool_rows += used;
     s.batches++;
-    if (nb == a.npk - p0 || nb >= 1024) rpp = std::max(1.0, (double)used / (double)nb);
+    if (nb == a.npk - p0 || nb >= 1024) {
+      rpp = std::max(1.0, (double)used / (double)nb);
+      most = std::max(most, rpp);
+    }
     if (nb >= 1024) sl.walk_per_peak = (double)(c[9] - before[9]) / (double)nb;
     std::memcpy(before, c, sizeof(c));
     p0 += nb;
   }
-  // the next call's estimate: the rows per peak of the whole call (the last
-  // batch's alone would be the small radii's, and the first batch of the next
-  // call would overflow the pool and run twice)
-  if (s.batches > 1) rpp = std::max(1.0, (double)s.pool_rows / (double)a.npk);
+  // the next call's estimate: the most rows per peak of any batch.  Lists come
+  // largest radius first, so with the last batch's or the whole call's mean the
+  // first batch of the next such call would overflow the pool and run twice
+  if (most > 0.0) sl.rows_per_peak[adaptive] = most;
   s.visits = c[0];
   for (int i = 0; i < 5; i++) s.dump[i] = c[1 + i];
   s.guard = c[6];

@@ -164,7 +164,7 @@ struct Slot {
   }
   DevBuf pft;                                       // ppb_peak_find_tile: unpacked (i, j, k), ipp, filter
   int gather_bps[2][2][2] = {};                      // gather blocks per SM by [comp][adaptive][ring]
-  double rows_per_peak[2] = {0.0, 0.0};             // pool rows per peak seen last, by adaptive
+  double rows_per_peak[2] = {0.0, 0.0};             // pool rows per peak of the last call's largest batch, by adaptive
   double walk_per_peak = 0.0;                       // collapse-walk steps per peak seen last
   ShellStats last_shell{};
   int64_t last_visits = 0, last_npk = 0;
