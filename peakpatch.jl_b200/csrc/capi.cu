@@ -478,9 +478,24 @@ TuneEntry ppb_ctx::tune_shells(Slot& sl, const ShellArgs& b0, bool comp, bool ad
     te.gather_tex = !(best < 0.99f * te.gather_ms[bi]);
   }
   // collapse: the size heuristic's width in list order unless another
-  // (width, order) is at least 3 % faster
+  // (width, order) is at least 3 % faster.  A warp per peak, the heuristic's
+  // choice for small batches, is none of the candidates and timed by itself
   const int wd = shell_collapse_width(b.npk, nsm, sl.walk_per_peak);
-  const int di = wd >= 4 ? 2 : wd - 1;   // a batch that is tuned is too large for a warp per peak
+  const int di = wd >= 4 ? 2 : wd - 1;
+  float dms = te.collapse_ms[di];
+  if (wd > 4) {
+    dms = 1e30f;
+    collapse_order(sl, b, false);
+    for (int round = 0; round < 2; round++) {
+      PPB_CUDA(cudaEventRecord(ev[0], s));
+      launch_shell_collapse(L, b, nsm, sl.walk_per_peak, 0);
+      PPB_CUDA(cudaEventRecord(ev[1], s));
+      PPB_CUDA(cudaEventSynchronize(ev[1]));
+      float ms = 0.f;
+      PPB_CUDA(cudaEventElapsedTime(&ms, ev[0], ev[1]));
+      dms = std::min(dms, ms);
+    }
+  }
   int ci = di, co = 0;
   for (int o = 0; o < 2; o++)
     for (int c = 0; c < 4; c++) {
@@ -488,7 +503,7 @@ TuneEntry ppb_ctx::tune_shells(Slot& sl, const ShellArgs& b0, bool comp, bool ad
       if (t < (co ? te.collapse_ordered_ms[ci] : te.collapse_ms[ci])) { ci = c; co = o; }
     }
   const float best = co ? te.collapse_ordered_ms[ci] : te.collapse_ms[ci];
-  if (best < 0.97f * te.collapse_ms[di]) {
+  if (best < 0.97f * dms) {
     te.collapse_threads = widths[ci];
     te.collapse_order = co == 1;
   } else {
