@@ -112,6 +112,7 @@ bool Slot::give_back_stub() {
 
 void Slot::release_buffers() {
   if (stream) PPB_CUDA(cudaStreamSynchronize(stream));
+  if (stream2) PPB_CUDA(cudaStreamSynchronize(stream2));
   drop_record_texture();
   release_stub();
   merge.release();
@@ -151,7 +152,7 @@ int Slot::lru_tile(int keep) const {
 uint64_t Slot::drop_tile(int n) {
   auto it = tiles.find(n);
   if (it == tiles.end()) return 0;
-  PPB_CUDA(cudaStreamSynchronize(stream));   // nothing of that size in flight
+  for (cudaStream_t s : {stream, stream2}) PPB_CUDA(cudaStreamSynchronize(s));   // nothing of that size in flight
   const uint64_t b = it->second->bytes();
   tiles.erase(it);
   tile_lru.erase(std::remove(tile_lru.begin(), tile_lru.end(), n), tile_lru.end());

@@ -563,15 +563,28 @@ void setup_run(Run& r, ppb_ctx* ctx, Slot& sl, const ppb_tile_params* p, const d
 }
 
 // the slot's second stream starts from here on / the slot's stream waits for
-// it; both legal while the slot's stream is being captured
-void fork(Slot& sl) {
-  PPB_CUDA(cudaEventRecord(sl.fork_ev, sl.stream));
-  PPB_CUDA(cudaStreamWaitEvent(sl.stream2, sl.fork_ev, 0));
-}
-void join(Slot& sl) {
-  PPB_CUDA(cudaEventRecord(sl.join_ev, sl.stream2));
-  PPB_CUDA(cudaStreamWaitEvent(sl.stream, sl.join_ev, 0));
-}
+// it; both legal while the slot's stream is being captured.  An exception
+// between them joins too: what follows on the slot's stream, a later call's
+// work on the same buffers included, never runs beside leftover work
+struct SecondStream {
+  Slot& sl;
+  bool open = false;
+  explicit SecondStream(Slot& s) : sl(s) {}
+  void fork() {
+    PPB_CUDA(cudaEventRecord(sl.fork_ev, sl.stream));
+    PPB_CUDA(cudaStreamWaitEvent(sl.stream2, sl.fork_ev, 0));
+    open = true;
+  }
+  void join() {
+    open = false;
+    PPB_CUDA(cudaEventRecord(sl.join_ev, sl.stream2));
+    PPB_CUDA(cudaStreamWaitEvent(sl.stream, sl.join_ev, 0));
+  }
+  ~SecondStream() {
+    if (open && cudaEventRecord(sl.join_ev, sl.stream2) == cudaSuccess)
+      cudaStreamWaitEvent(sl.stream, sl.join_ev, 0);
+  }
+};
 
 // phase 1 (Pipeline.jl:90-140, MultiTile.jl:157-194): Threefry noise -> R2C
 // -> sqrt(P) -> C2R = delta; delta_k = R2C(delta), projected Hermitian;
@@ -598,8 +611,9 @@ void fields_phase(Run& r, TileRes& T, int n, double box) {
   // 1LPT; on small grids beside 2LPT and the Laplacian, on the slot's second
   // stream
   const bool two = T.c2r3b && !r.plain;
+  SecondStream beside(*r.sl);
   if (two) {
-    fork(*r.sl);
+    beside.fork();
     const Launch L2{r.sl->stream2, L.count};
     float2* kb = T.kwb.as<float2>();
     launch_lpt1(L2, dkp, kb, n, box, inv_n3);
@@ -659,7 +673,7 @@ void fields_phase(Run& r, TileRes& T, int n, double box) {
     launch_hermitise(L, kw, n, 1);
     PPB_CUFFT(cufftExecC2R(T.c2r1, (cufftComplex*)kw, T.lapd.as<cufftReal>()));
   }
-  if (two) join(*r.sl);
+  if (two) beside.join();
 }
 
 // phase 2 (Pipeline.jl:144-196, MultiTile.jl:218-275): per filter, largest
@@ -726,6 +740,7 @@ int64_t peaks_phase(Run& r, TileRes& T, int n, double box, const std::vector<Win
       PPB_CUDA(cudaMemsetAsync(T.count.p, 0, 64, r.s));
       launch_window_tables(L, T.wtab.as<float>(), n, box, r.sl->filt_Rf.as<double>(), r.nfilt, p->wsmooth,
                            r.want_lap);
+      SecondStream beside(*r.sl);
       for (int f = 0; f < r.nfilt; f++) {
         const float* tab = T.wtab.as<float>() + (size_t)f * 2 * qn;
         if (twin && f % group == 0) PPB_CUDA(cudaMemcpyAsync(first, T.count.p, 4, cudaMemcpyDeviceToDevice, r.s));
@@ -751,10 +766,10 @@ int64_t peaks_phase(Run& r, TileRes& T, int n, double box, const std::vector<Win
           };
           const bool two = T.c2r1b && !r.plain, second = two && f % 2 == 1;
           if (two && f % 2 == 0 && f + 1 < r.nfilt) {
-            fork(*r.sl);
+            beside.fork();
             smooth(Launch{r.sl->stream2, L.count}, f + 1, T.kwb.as<float2>(), T.rwb.as<float>(), T.c2r1b, T.c2r2b);
           }
-          if (second) join(*r.sl);
+          if (second) beside.join();
           else smooth(L, f, kw, rw, T.c2r1, T.c2r2);
           const float* x = second ? T.rwb.as<float>() : rw;
           for (size_t t = 0; t < wins.size(); t++) {
