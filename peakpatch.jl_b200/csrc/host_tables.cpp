@@ -113,7 +113,7 @@ void build_shell_table(ShellTable& st, int nhunt) {
   // and smaller in the first groups, where most peaks of a tile stop (a group
   // is gathered whole, so its size is the truncation's grain): with
   // kFirstChunk cells in the first kFirstGroups groups the 384^3 tile visits
-  // 6.9e8 cells instead of 8.2e8 (8.20 -> 7.61 ms), while whole spheres of
+  // 7.1e8 cells instead of 8.2e8 (8.20 -> 7.61 ms), while whole spheres of
   // thousands of cells keep the larger chunks (200,000 peaks to 24 cells:
   // 5.32 ms with 24 throughout, 6.11 with 16, 5.36 so)
   const int csize = std::min(kChunkCells, std::max(4, 4 * ((total + 127) / 128)));

@@ -47,10 +47,10 @@ template <int SIGN> __device__ __forceinline__ float2 twid(float2 a, const float
   return fft::rot<SIGN>(a, w.x, w.y);
 }
 
-// k-space factors as unevaluated sums of two floats (about 47 bits), applied
+// k-space factors as unevaluated sums of two floats (43 bits and more), applied
 // with one rounding: the accuracy of a factor formed in FP64 without its
 // conversions and division (fields with 2LPT and Laplacian at 384^3: 6.92 ms
-// with factors rounded to float, 7.22 in FP64, 7.07 so)
+// with factors rounded to float, 7.22 in FP64, 6.98 so)
 struct Pair {
   float h, l;
 };
@@ -60,7 +60,8 @@ __device__ __forceinline__ Pair operator*(const Pair& a, float b) {
   return Pair{h, fmaf(a.l, b, fmaf(a.h, b, -h))};
 }
 __device__ __forceinline__ Pair over(const Pair& a, int q) {   // a / q, 0 < q < 2^24
-  const float r = __frcp_rn((float)q), e = r * fmaf(-(float)q, r, 1.f), h = a.h * r;
+  // r is within 2 ulp of 1 / q, r + e within 2^-43
+  const float r = __fdividef(1.f, (float)q), e = r * fmaf(-(float)q, r, 1.f), h = a.h * r;
   return Pair{h, fmaf(a.h, e, fmaf(a.l, r, fmaf(a.h, r, -h)))};
 }
 __device__ __forceinline__ float apply(float x, const Pair& s) { return fmaf(x, s.h, x * s.l); }
@@ -574,6 +575,9 @@ template <int N> void rows_n(Launch L, const float2* w, float* out, const float2
   PPB_LAUNCHED(*L.count);
 }
 
+// every multiple of 16 up to 384, the largest tile of the workloads, and the
+// two larger sizes of the fused x pass (k_xpeak.cu); a size adds about 0.3 MB
+// to the library and 5 s to the build, and the others take cuFFT
 #define PPB_FFT_SIZES(X) \
   X(4) X(5) X(6) X(7) X(8) X(9) X(10) X(11) X(12) X(13) X(14) X(15) X(16) X(17) X(18) X(19) X(20) X(21) X(22) \
   X(23) X(24) X(28) X(32)

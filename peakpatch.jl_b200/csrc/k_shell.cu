@@ -1053,10 +1053,14 @@ __device__ __forceinline__ uint32_t spread3(uint32_t v) {
 // axis), so that peaks whose spheres overlap (of any filter) are gathered
 // close in time and share cached records.  The two bits above it put the
 // peaks of many cells first (a warp takes a peak whole, and one begun last
-// keeps the launch waiting): 200,000 peaks to 24 cells 5.42 -> 4.93 ms, four
-// lightcone tiles of 192^3 5.06 -> 4.89.  Not in small batches, where the
-// longest are peaks whose crossing no bound foresees, and would start later
-// (23,070 peaks of a 128^3 tile 0.26 -> 0.32 ms)
+// keeps the launch waiting).  Random radii to 24 cells, gather without -> with:
+// 50,000 peaks 2.09 -> 2.08 ms (below the line, no classes), 100,000 3.21 ->
+// 2.97, 200,000 5.40 -> 4.92, 800,000 18.4 -> 18.1; tiles of 192^3 (107,609
+// peaks) 1.04 -> 0.99, 256^3 2.14 -> 2.09, 320^3 4.53 -> 4.55, and 384^3
+// (861,595) 7.13 -> 7.25, where the classes cost more shared records than the
+// end of the launch gains.  Not in small batches, where the longest are peaks
+// whose crossing no bound foresees, and would start later (23,070 peaks of a
+// 128^3 tile 0.26 -> 0.32 ms)
 constexpr int kLongCells = 2048, kLongPeaks = 65536;
 __global__ void geo_kernel(ShellArgs a, uint32_t* key, int32_t* idx) {
   const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;

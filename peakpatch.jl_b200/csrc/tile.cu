@@ -290,9 +290,12 @@ TileRes::~TileRes() {
 }
 
 // largest grid whose transforms take a second stream: up to here a kernel of
-// one field leaves part of the device idle (run_tile 142^3 4.00 -> 3.64 ms,
-// fields 142^3 1.69 -> 1.56 with phi_33 from the trace, 128^3 tile 1.94 ->
-// 1.87); the kernels of a 192^3 field fill it
+// one field leaves part of the device idle.  Tiles, one stream -> two (device
+// ms): 96^3 1.09 -> 1.00, 112^3 1.32 -> 1.21, 128^3 1.33 -> 1.26, 142^3 5.95
+// -> 5.68, 150^3 3.01 -> 2.86, 160^3 2.31 -> 2.19, 176^3 2.75 -> 2.60, 256^3
+// 6.35 -> 6.35; 192^3 3.41 -> 3.40 (the fused filter bank has one stream).
+// The line stays below 176^3 for memory: the second set of buffers is 20
+// bytes a cell
 constexpr int kTwoStreams = 160;
 
 // the second stream's smoothed field, and its full twin where there is one
@@ -444,17 +447,15 @@ static uint64_t plan_work_bytes(int n) {
   std::lock_guard<std::mutex> lk(mu);
   auto it = known.find(n);
   if (it != known.end()) return it->second;
-  auto work = [&](cufftType t, int batch) {
+  auto work = [&](int batch) {   // no plan of fewer transforms needs more
     int dims[3] = {n, n, n};
     size_t w = 0;
-    const cufftResult r = cufftEstimateMany(3, dims, nullptr, 1, 0, nullptr, 1, 0, t, batch, &w);
+    const cufftResult r = cufftEstimateMany(3, dims, nullptr, 1, 0, nullptr, 1, 0, CUFFT_C2R, batch, &w);
     if (r == CUFFT_SUCCESS) return (uint64_t)w;
     return (uint64_t)(batch + 1) * 16 * (n / 2 + 1) * n * n;   // the most of any size: two half spectra per transform and two more
   };
-  const uint64_t two = std::max(work(CUFFT_C2R, 1), work(CUFFT_C2R, 3));
-  uint64_t one = std::max(two, work(CUFFT_R2C, 1));
-  if (!fft_supported(n)) one = std::max(one, work(CUFFT_C2R, 5));
-  return known[n] = one + two;
+  const uint64_t three = work(3);
+  return known[n] = (fft_supported(n) ? three : work(5)) + three;
 }
 
 uint64_t tile_bytes_estimate(int nn) {
