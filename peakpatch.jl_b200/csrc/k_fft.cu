@@ -22,9 +22,10 @@
 // spectrum read or written the passes move 3 + 7 + 6.5 + 2 + 3 + 5 + 4.5 = 31;
 // separate transforms (multiply, Hermitian projection, three passes each)
 // move about 110.  Measured at 384^3 (231 MB per half spectrum): col_kernel
-// 4.0-4.4 TB/s of HBM traffic, src2_rows_kernel 0.71 ms (2.1 TB/s; 15 warps
-// per SM at 128 registers), mid_kernel 0.29 ms, row_kernel 3.2 TB/s; 2LPT
-// with the Laplacian 6.4 -> 2.6 ms.
+// 4.0-4.4 TB/s of HBM traffic in the y passes (the z passes are bound by
+// instructions, the factor of every mode), src2_rows_kernel 0.74 ms (2.1
+// TB/s; 15 warps per SM at 128 registers), mid_kernel 0.30 ms, row_kernel 3.2
+// TB/s; 2LPT with the Laplacian 6.4 -> 2.7 ms.
 #include <cstdint>
 
 #include "ppb_fft.cuh"

@@ -26,8 +26,8 @@
 // the next step's start and the two midpoint evaluations share theirs, so
 // both are evaluated once, side by side, at the step's start.
 // Nodes are taken by ascending F, the longest integrations first.  One thread
-// per node: 307 ms for the 50 x 20 x 20 table; this: 174 ms,
-// 107 ms of it the longest node's latency (the same bits).
+// per node: 307 ms a call for the 50 x 20 x 20 table; this: 163 ms, 107 ms of
+// it the longest node's latency (the same bits).
 //
 // Bit-exactness with the CPU oracle: this file is compiled without
 // multiply-add contraction (-fmad=false), so that every +, -, *, / and sqrt

@@ -632,7 +632,7 @@ void fields_phase(Run& r, TileRes& T, int n, double box) {
   }
   // psi2 and the Laplacian feed no collapse decision: for the sizes of
   // k_fft.cu they take the fused transforms (fields with 2LPT and Laplacian,
-  // all transforms by cuFFT -> these fused: 384^3 11.0 -> 7.2 ms, 352^3 9.9
+  // all transforms by cuFFT -> these fused: 384^3 11.0 -> 7.0 ms, 352^3 9.9
   // -> 6.2); elsewhere, and on the plain path, a full transform per field.
   // delta and psi keep cuFFT's rounding, on which the peak list depends
   const bool fused = !r.plain && fft_supported(n);
